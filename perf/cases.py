@@ -171,21 +171,16 @@ def _zero_gradients(model):
     return [id(p) in zero for p in model.parameters()]
 
 
-def prepare(case, seed):
-    torch_ops.load()
+def _make(case, seed):
+    """The plain model, inputs and targets of a case, on the GPU, from the seed alone."""
     torch.manual_seed(seed)
-    state = dict(case)
+    b, y = case["batch"], None
     with torch.device("cuda"):
         if case["kind"] == "cnn":
             model = _network(case).to(memory_format=torch.channels_last)
-            images = torch.randn(case["batch"], 3, case["image"], case["image"])
-            state["x"] = images.contiguous(memory_format=torch.channels_last)
+            x = torch.randn(b, 3, case["image"], case["image"]).contiguous(memory_format=torch.channels_last)
             if case["train"]:
-                state["params"], state["zero"] = list(model.parameters()), _zero_gradients(model)
-                state["y"] = torch.randint(0, CLASSES, (case["batch"],))
-                state["model"] = torch_ops.prepare_training(model)
-                state["opt"] = optim.SGD(state["params"], lr=0.01, momentum=0.9)
-                state["loss"] = nn.CrossEntropyLoss()
+                y = torch.randint(0, CLASSES, (b,))
             else:
                 for m in model.modules():
                     if isinstance(m, nn.BatchNorm2d):   # statistics and scales as a trained network has them
@@ -193,18 +188,31 @@ def prepare(case, seed):
                         nn.init.normal_(m.bias, 0.0, 0.1)
                         m.running_mean.normal_(0.0, 0.2)
                         m.running_var.uniform_(0.5, 1.5)
-                state["model"] = torch_ops.prepare_inference(model)
         else:
-            bert = case["model"] == "bert"
+            bert, s = case["model"] == "bert", case["seq"]
             cfg = dict(BERT if bert else LM, layers=case["layers"])
             model = (BertQA if bert else DecoderLM)(cfg).to(torch.bfloat16)
-            b, s = case["batch"], case["seq"]
-            state["x"] = torch.randint(0, 30522 if bert else cfg["vocab"], (b, s))
-            state["model"] = model.train(case["train"])
+            x = torch.randint(0, 30522 if bert else cfg["vocab"], (b, s))
             if case["train"]:
-                state["params"], state["zero"] = list(model.parameters()), _zero_gradients(model)
-                state["y"] = torch.randint(0, s, (2 * b,)) if bert else torch.randint(0, cfg["vocab"], (b * s,))
-                state["opt"] = optim.AdamW(state["params"], lr=3e-5 if bert else 3e-4)
+                y = torch.randint(0, s, (2 * b,)) if bert else torch.randint(0, cfg["vocab"], (b * s,))
+    return model.train(case["train"]), x, y
+
+
+def prepare(case, seed):
+    torch_ops.load()
+    state = dict(case)
+    model, state["x"], state["y"] = _make(case, seed)
+    if case["train"]:
+        state["params"], state["zero"] = list(model.parameters()), _zero_gradients(model)
+    if case["kind"] == "text":
+        state["model"] = model
+        if case["train"]:
+            state["opt"] = optim.AdamW(state["params"], lr=3e-5 if case["model"] == "bert" else 3e-4)
+    elif case["train"]:
+        state["model"], state["loss"] = torch_ops.prepare_training(model), nn.CrossEntropyLoss()
+        state["opt"] = optim.SGD(state["params"], lr=0.01, momentum=0.9)
+    else:
+        state["model"] = torch_ops.prepare_inference(model)
     return state
 
 
@@ -274,6 +282,71 @@ def work(case):
         return {"bytes": 2.0 * (layers * per_layer + head + rows_read * h + logits), "flops": flops}
     # weights and both moments are read and written, gradients written; logits are kept from forward to backward
     return {"bytes": 2.0 * (7 * (layers * per_layer + head + table) + 2 * logits), "flops": 3.0 * flops}
+
+
+def _text_exact(model, x, causal):
+    """The logits, from the weights of a float64 copy of a language model."""
+    p = dict(model.named_parameters())
+    heads, s = model.layers[0].heads, x.shape[1]
+
+    def linear(h, name):
+        return F.linear(h, p[name + ".weight"], p[name + ".bias"])
+
+    def norm(h, name, eps):
+        return F.layer_norm(h, h.shape[-1:], p[name + ".weight"], p[name + ".bias"], eps)
+
+    h = p["word.weight"][x] + p["pos.weight"][:s]
+    if not causal:
+        h = norm(h + p["typ.weight"][0], "ln", 1e-12)
+    future = torch.ones(s, s, dtype=torch.bool, device=x.device).triu(1)
+    for i in range(len(model.layers)):
+        n = "layers.%d." % i
+        q, k, v = linear(h, n + "qkv").view(*x.shape, 3, heads, -1).permute(2, 0, 3, 1, 4)
+        scores = q @ k.transpose(-1, -2) / math.sqrt(q.shape[-1])
+        if causal:
+            scores = scores.masked_fill(future, -math.inf)
+        context = (scores.softmax(-1) @ v).transpose(1, 2).flatten(2)
+        h = norm(h + linear(context, n + "out"), n + "ln1", 1e-12)
+        h = norm(h + linear(F.gelu(linear(h, n + "fc1")), n + "fc2"), n + "ln2", 1e-12)
+    if causal:
+        return F.linear(norm(h, "ln", 1e-5), p["head.weight"])
+    return linear(h, "qa")
+
+
+def exact(case, seed):
+    model, x, y = _make(case, seed)
+    zero = _zero_gradients(model)
+    model = model.double()
+    with torch.set_grad_enabled(case["train"]):
+        if case["kind"] == "cnn":
+            logits = model(x.double())
+        else:
+            logits = _text_exact(model, x, case["model"] == "lm")
+    if not case["train"]:
+        return logits
+    if case["kind"] == "cnn":
+        loss = F.cross_entropy(logits, y)
+    elif case["model"] == "bert":
+        loss = 2.0 * F.cross_entropy(logits.permute(2, 0, 1).reshape(-1, case["seq"]), y)
+    else:
+        loss = F.cross_entropy(logits.flatten(0, 1), y)
+    loss.backward()
+    params, text = list(model.parameters()), case["kind"] == "text"
+    # In BERT, the gradient of the shift before the last norm cancels over the positions almost as far as the gradients that are
+    # left out, and bfloat16 leaves it 0.16 off.
+    poor = id(model.layers[-1].fc2.bias) if text and case["model"] == "bert" else None
+    out = {"loss": loss.detach(), "grads": [None if id(p) == poor else p.grad for p, z in zip(params, zero) if not z]}
+    if 2 * len(params) + 1 <= 64:
+        # the first step of AdamW moves a weight by the sign of its gradient, and a vector that starts at zero is that alone
+        lr = (3e-5 if case["model"] == "bert" else 3e-4) if text else 0.01
+        out["weights"] = []
+        for p in params:
+            if text:
+                new = p.detach() * (1 - lr * 1e-2) - lr * p.grad / (p.grad.abs() + 1e-8) if p.dim() > 1 and p.grad is not None else None
+            else:
+                new = p.detach() - lr * p.grad
+            out["weights"].append(new)
+    return out
 
 
 def tolerance(case):
