@@ -89,6 +89,8 @@ class BertLayer(nn.Module):
         if d == 64 and s <= 384 and x.dtype == torch.bfloat16 and FUSED_ATTENTION:
             # scores, softmax and the context product in one kernel, read straight from the projection's output
             ctx = ops.attention(qkv.view(b, s, 3 * h), self.heads, 1.0 / math.sqrt(d), causal)
+        elif d == 64 and s % 8 == 0 and x.dtype == torch.bfloat16 and FUSED_ATTENTION:
+            ctx = ops.attention_long(qkv.view(b, s, 3 * h), self.heads, 1.0 / math.sqrt(d), causal)
         else:
             qkv = qkv.view(b, s, 3, self.heads, d)
             q = qkv[:, :, 0].permute(0, 2, 1, 3).reshape(b * self.heads, s, d).contiguous()

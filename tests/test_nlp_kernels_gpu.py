@@ -172,6 +172,25 @@ def test_fused_attention_matches_float64(tops, B, S, H, causal):
     assert O.rel_err(ctx, want) < 2e-2
 
 
+@pytest.mark.parametrize("B,S,H,causal,spread", [(2, 512, 16, True, 1.0), (1, 392, 3, False, 1.0), (1, 8, 2, True, 1.0), (3, 1032, 2, True, 4.0),
+                                                 (1, 648, 5, False, 6.0)])
+@pytest.mark.parametrize("scale", [0.125, -0.125])
+def test_long_attention_matches_float64(tops, B, S, H, causal, spread, scale):
+    """The same for long sequences: 64-key steps with a running maximum.  `spread` widens the scores so that a row's maximum
+    outgrows the reference maximum by more than 2^8 between steps and sums and output are rescaled; a negative scale turns the
+    order of the scores round."""
+    from orion_b200 import kernels
+    torch.manual_seed(40 + S)
+    qkv = (torch.randn(B, S, 3 * H * 64, device="cuda") * spread).to(torch.bfloat16)
+    ctx = tops.attention_long(qkv, H, scale, causal).view(B, S, H, 64)
+    assert kernels.read_status() == 0
+    q, k, v = qkv.double().cpu().view(B, S, 3, H, 64).permute(2, 0, 3, 1, 4)
+    # (the stock function takes the square root of its scale)
+    want = F.scaled_dot_product_attention(q * scale, k, v, is_causal=causal, scale=1.0).permute(0, 2, 1, 3)
+    # probabilities and output are rounded to bfloat16 (2^-9 each, relative to values of at most the largest |v|)
+    assert O.rel_err(ctx, want) < 1e-2
+
+
 # ---------------------------------------------------------------------------------------------- training on the own GEMM
 @pytest.mark.parametrize("rows,K,N,bias,res", [(3072, 768, 2304, True, False), (3072, 768, 768, True, True), (520, 256, 136, False, True),
                                                (64, 3072, 768, True, True), (8192, 1024, 1024, False, False)])
