@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
     uint8_t* v_s = k_s + AT_RING * AT_KV_BYTES;
     uint8_t* p_s = v_s + AT_RING * AT_KV_BYTES;
     AttnCtl* ctl = reinterpret_cast<AttnCtl*>(p_s + AT_P_BYTES);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp_index(), lane = tid & 31;
 
     if (tid == 0) {
         mbar_init(&ctl->q_full, 1);
@@ -124,76 +124,85 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
     const int items = p.last;
 
     if (warp == 4) {
-        // ------------------------------------------------------------ TMA
-        if (lane == 0) {
-            uint32_t n = 0, local = 0;   // key steps, items
-            bool dead = false;
-            for (int item = p.first + blockIdx.x; item < items && !dead; item += gridDim.x, local++) {
-                const AttnItem it(p, item);
-                if (!mbar_wait(&ctl->q_empty, (local & 1u) ^ 1u, abort_flag)) { attn_give_up(ctl, p.status, OB200_ERR_WAIT_EMPTY); break; }
+        // ------------------------------------------------------------ TMA (the warp as one, see elect_one)
+        uint32_t n = 0, local = 0;   // key steps, items
+        bool dead = false;
+        for (int item = p.first + blockIdx.x; item < items && !dead; item += gridDim.x, local++) {
+            const AttnItem it(p, item);
+            dead = !mbar_wait_warp(&ctl->q_empty, (local & 1u) ^ 1u, abort_flag);
+            if (dead) break;
+            if (elect_one()) {
                 mbar_arrive_expect_tx(&ctl->q_full, AT_Q_BYTES);
 #pragma unroll
                 for (int g = 0; g < 2; g++)
                     tma_load_tile_4d(smem_u32(q_s + g * 64 * 128), p.tmap, &ctl->q_full, 0, it.h, it.qt * AT_QROWS + g * 64, it.b);
-                for (int t = 0; t < it.steps; t++, n++) {
-                    const uint32_t s = n % AT_RING, ph = (n / AT_RING) & 1u;
-                    if (!mbar_wait(&ctl->k_empty[s], ph ^ 1u, abort_flag)) { dead = true; break; }
+            }
+            __syncwarp();
+            for (int t = 0; t < it.steps; t++, n++) {
+                const uint32_t s = n % AT_RING, ph = (n / AT_RING) & 1u;
+                dead = !mbar_wait_warp(&ctl->k_empty[s], ph ^ 1u, abort_flag);
+                if (dead) break;
+                if (elect_one()) {
                     mbar_arrive_expect_tx(&ctl->k_full[s], AT_KV_BYTES);
                     tma_load_tile_4d(smem_u32(k_s + s * AT_KV_BYTES), p.tmap, &ctl->k_full[s], 0, p.H + it.h, t * AT_KEYS, it.b);
-                    if (!mbar_wait(&ctl->v_empty[s], ph ^ 1u, abort_flag)) { dead = true; break; }
+                }
+                __syncwarp();
+                dead = !mbar_wait_warp(&ctl->v_empty[s], ph ^ 1u, abort_flag);
+                if (dead) break;
+                if (elect_one()) {
                     mbar_arrive_expect_tx(&ctl->v_full[s], AT_KV_BYTES);
                     tma_load_tile_4d(smem_u32(v_s + s * AT_KV_BYTES), p.tmap, &ctl->v_full[s], 0, 2 * p.H + it.h, t * AT_KEYS, it.b);
                 }
-                if (dead) attn_give_up(ctl, p.status, OB200_ERR_WAIT_EMPTY);
+                __syncwarp();
             }
         }
+        if (dead) attn_give_up(ctl, p.status, OB200_ERR_WAIT_EMPTY);
     } else if (warp == 5) {
-        // ------------------------------------------------------------ MMA issue
+        // ------------------------------------------------------------ MMA issue (the warp as one)
         // S(n) = Q . K(n)^T is issued as soon as the softmax warps have the scores of step n-1 in registers, before P(n-1) is
         // ready, so it runs under their exponentials; O += P(n) . V(n) follows when P(n) is in shared memory.
-        if (lane == 0) {
-            const uint32_t idesc_s = umma_idesc(1, AT_QROWS, AT_KEYS), idesc_o = umma_idesc(1, AT_QROWS, AT_D) | UMMA_IDESC_B_MN;
-            const uint64_t qd = umma_desc_sw128(smem_u32(q_s)), pd = umma_desc_sw128(smem_u32(p_s));
-            uint32_t n = 0, local = 0;
-            bool dead = false;
-            auto scores = [&](uint32_t i) {
-                const uint32_t s = i % AT_RING;
-                if (!mbar_wait(&ctl->k_full[s], (i / AT_RING) & 1u, abort_flag)) return false;
-                if (i > 0 && !mbar_wait(&ctl->s_free, (i - 1) & 1u, abort_flag)) return false;
-                tc_fence_after_sync();
+        const uint32_t idesc_s = umma_idesc(1, AT_QROWS, AT_KEYS), idesc_o = umma_idesc(1, AT_QROWS, AT_D) | UMMA_IDESC_B_MN;
+        const uint64_t qd = umma_desc_sw128(smem_u32(q_s)), pd = umma_desc_sw128(smem_u32(p_s));
+        // V lies as [key][64]: MN-major, atoms of 8 keys x 128 bytes, 1024 bytes apart along the reduction
+        const uint64_t v_bits = ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+        uint32_t n = 0, local = 0;
+        bool dead = false;
+        auto scores = [&](uint32_t i, bool last) {
+            const uint32_t s = i % AT_RING;
+            if (!mbar_wait_warp(&ctl->k_full[s], (i / AT_RING) & 1u, abort_flag)) return false;
+            if (i > 0 && !mbar_wait_warp(&ctl->s_free, (i - 1) & 1u, abort_flag)) return false;
+            tc_fence_after_sync();
+            if (elect_one()) {
                 const uint64_t kd = umma_desc_sw128(smem_u32(k_s + s * AT_KV_BYTES));
 #pragma unroll
                 for (int ks = 0; ks < AT_D / 16; ks++) umma_f16(t_s, qd + (uint64_t)ks * 2, kd + (uint64_t)ks * 2, idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(&ctl->k_empty[s]);
+                if (last) umma_commit(&ctl->q_empty);   // every product with this Q tile is issued
                 umma_commit(&ctl->s_full);
-                return true;
-            };
-            for (int item = p.first + blockIdx.x; item < items && !dead; item += gridDim.x, local++) {
-                const AttnItem it(p, item);
-                dead = !mbar_wait(&ctl->q_full, local & 1u, abort_flag) || !scores(n);
-                for (int t = 0; t < it.steps && !dead; t++, n++) {
-                    if (t + 1 < it.steps) {
-                        if (!scores(n + 1)) { dead = true; break; }
-                    } else {
-                        umma_commit(&ctl->q_empty);   // every product with this Q tile is issued
-                    }
-                    const uint32_t s = n % AT_RING;
-                    if (!mbar_wait(&ctl->v_full[s], (n / AT_RING) & 1u, abort_flag) || !mbar_wait(&ctl->p_full, n & 1u, abort_flag)) { dead = true; break; }
-                    tc_fence_after_sync();
+            }
+            __syncwarp();
+            return true;
+        };
+        for (int item = p.first + blockIdx.x; item < items && !dead; item += gridDim.x, local++) {
+            const AttnItem it(p, item);
+            dead = !mbar_wait_warp(&ctl->q_full, local & 1u, abort_flag) || !scores(n, it.steps == 1);
+            for (int t = 0; t < it.steps && !dead; t++, n++) {
+                if (t + 1 < it.steps && !scores(n + 1, t + 2 == it.steps)) { dead = true; break; }
+                const uint32_t s = n % AT_RING;
+                if (!mbar_wait_warp(&ctl->v_full[s], (n / AT_RING) & 1u, abort_flag) || !mbar_wait_warp(&ctl->p_full, n & 1u, abort_flag)) { dead = true; break; }
+                tc_fence_after_sync();
+                if (elect_one()) {
+                    const uint64_t vd = umma_desc_mn(v_bits, smem_u32(v_s + s * AT_KV_BYTES));
 #pragma unroll
-                    for (int ks = 0; ks < AT_KEYS / 16; ks++) {
-                        // V lies as [key][64]: MN-major, atoms of 8 keys x 128 bytes, 1024 bytes apart along the reduction
-                        const uint32_t v_addr = smem_u32(v_s + s * AT_KV_BYTES) + (uint32_t)ks * 2048u;
-                        const uint64_t vd = (uint64_t)((v_addr & 0x3FFFF) >> 4) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
-                                            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-                        umma_f16(t_o, pd + (uint64_t)ks * 2, vd, idesc_o, (t > 0 || ks > 0) ? 1u : 0u);
-                    }
+                    for (int ks = 0; ks < AT_KEYS / 16; ks++)
+                        umma_f16(t_o, pd + (uint64_t)ks * 2, vd + (uint64_t)ks * (2048 >> 4), idesc_o, ks > 0 ? 1u : (t > 0 ? 1u : 0u));
                     umma_commit(&ctl->v_empty[s]);
                     umma_commit(&ctl->o_full);
                 }
+                __syncwarp();
             }
-            if (dead) attn_give_up(ctl, p.status, OB200_ERR_WAIT_FULL);
         }
+        if (dead) attn_give_up(ctl, p.status, OB200_ERR_WAIT_FULL);
     } else {
         // ------------------------------------------------------------ softmax: thread r owns query row q0 + r (tensor-memory lane r)
         const int r = warp * 32 + lane;

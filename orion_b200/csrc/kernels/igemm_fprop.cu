@@ -12,7 +12,10 @@
 // tiles of 128 x BN.  Warp roles:
 //   warps 0-3   epilogue: tcgen05.ld the fp32 accumulator, apply scale/shift,
 //               residual and ReLU, store NHWC rows
-//   warp  4     allocates TMEM, one lane issues tcgen05.mma and tcgen05.commit
+//   warp  4     allocates TMEM, issues tcgen05.mma and tcgen05.commit: the warp runs the loop as one and an elected lane
+//               issues, which keeps the operands in uniform registers (elect_one).  From a lane-0 branch the issue itself bound
+//               every tile at about 100 cycles per MMA (3x3 64->64 at 56 x 56, batch 4: 1155 cycles per k-block of twelve
+//               MMAs; now 880, bound by the splitters; ResNet-50 batch 4 request 1200 -> 1071 us)
 //   warps 5-8   splitters (fp32 only): split the raw operand rows in shared memory into
 //               TF32 high parts (in place) and exact remainders (second buffer)
 //   warps 9-16  producers: cp.async 16-byte copies of one
@@ -312,6 +315,10 @@ __device__ __forceinline__ bool timed_wait(uint64_t* bar, uint32_t parity, volat
     acc += clock64() - t0;
     return ok;
 }
+// For roles that a converged warp runs as one (the answer is the same for all its lanes).
+__device__ __forceinline__ bool timed_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long& acc) {
+    return __all_sync(0xffffffffu, timed_wait(bar, parity, abort_flag, acc));
+}
 
 // Position in the ring of operand stages: stage index and the parity of the number of completed laps.
 struct RingPos {
@@ -399,7 +406,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + C::RING_BYTES + C::EPI_BYTES);
 
     const int tid = threadIdx.x;
-    const int warp = tid >> 5;
+    const int warp = uniform_warp_index();
     const int lane = tid & 31;
     constexpr int stages = C::STAGES;
     constexpr int stage_bytes = C::STAGE_BYTES;
@@ -617,84 +624,84 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         }
         if (p.debug && blockIdx.x == 0 && tid == 0) p.debug[0] = waited;
     } else if (warp == MMA_WARP) {
-        // ------------------------------------------------------------ MMA issue
-        if (lane == 0) {
-            // A TMA-fed filter gradient keeps both operands the way they lie in memory (pixel-major, i.e.
-            // MN-major for this GEMM); everything else stages K-major rows.
-            const bool mn_major = p.mode == 1 && p.use_tma;
-            const uint32_t idesc = umma_idesc(sizeof(T) == 4 ? 2 : 1, BM, BN) | (mn_major ? (UMMA_IDESC_A_MN | UMMA_IDESC_B_MN) : 0u);
-            const uint64_t kstep = mn_major ? (1024 >> 4) : (32 >> 4);   // descriptor address advance per k-step of 8 (16 for bf16)
-            RingPos ring;
-            int local = 0;
-            bool dead = false;
-            long long waited2 = 0;
-            const bool cross = ATMEM && p.cross_acc != 0;
-            WorkIter work(p, tiles);
-            Seg seg;
-            for (; !dead && work.next(seg); local++) {
-                const int kb_begin = seg.kb_begin, kb_end = seg.kb_end;
-                const int ab = cross ? 0 : (local & 1);
-                const uint32_t acc_use = cross ? (uint32_t)local : (uint32_t)(local >> 1);
-                if (!timed_wait(&ctl->tmem_empty[ab], (acc_use & 1u) ^ 1u, abort_flag, waited2)) {
-                    if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_EMPTY); }
+        // ------------------------------------------------------------ MMA issue (the warp as one, see elect_one)
+        // A TMA-fed filter gradient keeps both operands the way they lie in memory (pixel-major, i.e.
+        // MN-major for this GEMM); everything else stages K-major rows.
+        const bool mn_major = !ATMEM && p.mode == 1 && p.use_tma;
+        const uint32_t idesc = umma_idesc(sizeof(T) == 4 ? 2 : 1, BM, BN) | (mn_major ? (UMMA_IDESC_A_MN | UMMA_IDESC_B_MN) : 0u);
+        const uint64_t kstep = mn_major ? (1024 >> 4) : (32 >> 4);   // descriptor address advance per k-step of 8 (16 for bf16)
+        // operand descriptor above the address
+        const uint64_t desc_bits = mn_major ? p.mn_desc_bits : umma_desc_sw128(0);
+        RingPos ring;
+        int local = 0;
+        bool dead = false;
+        long long waited2 = 0;
+        const bool cross = ATMEM && p.cross_acc != 0;
+        WorkIter work(p, tiles);
+        Seg seg;
+        for (; !dead && work.next(seg); local++) {
+            const int kb_begin = seg.kb_begin, kb_end = seg.kb_end;
+            const int ab = cross ? 0 : (local & 1);
+            const uint32_t acc_use = cross ? (uint32_t)local : (uint32_t)(local >> 1);
+            if (!timed_wait_warp(&ctl->tmem_empty[ab], (acc_use & 1u) ^ 1u, abort_flag, waited2)) {
+                if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_EMPTY); }
+                break;
+            }
+            tc_fence_after_sync();
+            const uint32_t d = tmem_base + ab * BN;
+            // cross terms: into the main accumulator, or into one of their own (columns BN..2BN)
+            const uint32_t dx = cross ? tmem_base + BN : d;
+            for (int kb = kb_begin; kb < kb_end; kb++, ring.advance(stages)) {
+                const int s = ring.s;
+                // fp32: operands are ready when the splitters are done; bf16: when the copies have landed
+                if (!timed_wait_warp(C::kSplit ? &ctl->full[s] : &ctl->raw_full[s], ring.ph, abort_flag, waited)) {
+                    if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
+                    dead = true;
                     break;
                 }
+                if (!C::kSplit) fence_proxy_async_smem();   // cp.async wrote through the generic proxy
                 tc_fence_after_sync();
-                const uint32_t d = tmem_base + ab * BN;
-                for (int kb = kb_begin; kb < kb_end; kb++, ring.advance(stages)) {
-                    const int s = ring.s;
-                    // fp32: operands are ready when the splitters are done; bf16: when the copies have landed
-                    if (!timed_wait(C::kSplit ? &ctl->full[s] : &ctl->raw_full[s], ring.ph, abort_flag, waited)) {
-                        if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
-                        dead = true;
-                        break;
-                    }
-                    if (!C::kSplit) fence_proxy_async_smem();   // cp.async wrote through the generic proxy
-                    tc_fence_after_sync();
-                    const uint32_t base = smem_u32(smem + s * stage_bytes);
+                const uint32_t base = smem_u32(smem + s * stage_bytes);
+                const uint32_t first = kb > kb_begin ? 1u : 0u;   // 0: the k-block's first product overwrites its accumulator
+                const uint32_t first_hh = cross ? first : 1u;
+                if (elect_one()) {
+                    const uint64_t a_hi = umma_desc_mn(desc_bits, base), b_hi = umma_desc_mn(desc_bits, base + b_off);
                     if (C::kSplit) {
-                        const uint64_t a_hi = mn_major ? umma_desc_mn(p.mn_desc_bits, base) : umma_desc_sw128(base);
-                        const uint64_t a_lo = mn_major ? umma_desc_mn(p.mn_desc_bits, base + C::A_BYTES) : umma_desc_sw128(base + C::A_BYTES);
-                        const uint64_t b_hi = mn_major ? umma_desc_mn(p.mn_desc_bits, base + b_off) : umma_desc_sw128(base + b_off);
-                        const uint64_t b_lo = mn_major ? umma_desc_mn(p.mn_desc_bits, base + b_off + C::B_BYTES)
-                                                       : umma_desc_sw128(base + b_off + C::B_BYTES);
+                        const uint64_t a_lo = umma_desc_mn(desc_bits, base + C::A_BYTES);
+                        const uint64_t b_lo = umma_desc_mn(desc_bits, base + b_off + C::B_BYTES);
                         if (ATMEM) {
                             const uint32_t ta_hi = tmem_base + C::A_TMEM_COL0 + s * 64, ta_lo = ta_hi + 32;
 #pragma unroll
                             for (int ks = 0; ks < 4; ks++) {
-                                const uint64_t o = (uint64_t)ks * kstep;
-                                const uint32_t first = (kb > kb_begin || ks > 0) ? 1u : 0u;
-                                // cross terms: into the main accumulator, or into one of their own (columns BN..2BN)
-                                const uint32_t dx = cross ? tmem_base + BN : d;
-                                umma_tf32_ts(dx, ta_lo + ks * 8, b_hi + o, idesc, first);
+                                const uint64_t o = (uint64_t)ks * (32 >> 4);
+                                umma_tf32_ts(dx, ta_lo + ks * 8, b_hi + o, idesc, ks > 0 ? 1u : first);
                                 umma_tf32_ts(dx, ta_hi + ks * 8, b_lo + o, idesc, 1u);
-                                umma_tf32_ts(d, ta_hi + ks * 8, b_hi + o, idesc, cross ? first : 1u);
+                                umma_tf32_ts(d, ta_hi + ks * 8, b_hi + o, idesc, ks > 0 ? 1u : first_hh);
                             }
                         } else {
 #pragma unroll
                             for (int ks = 0; ks < 4; ks++) {
                                 const uint64_t o = (uint64_t)ks * kstep;
-                                umma_tf32(d, a_lo + o, b_hi + o, idesc, (kb > kb_begin || ks > 0) ? 1u : 0u);
+                                umma_tf32(d, a_lo + o, b_hi + o, idesc, ks > 0 ? 1u : first);
                                 umma_tf32(d, a_hi + o, b_lo + o, idesc, 1u);
                                 umma_tf32(d, a_hi + o, b_hi + o, idesc, 1u);
                             }
                         }
                     } else {
-                        const uint64_t a = mn_major ? umma_desc_mn(p.mn_desc_bits, base) : umma_desc_sw128(base);
-                        const uint64_t b = mn_major ? umma_desc_mn(p.mn_desc_bits, base + C::A_BYTES) : umma_desc_sw128(base + C::A_BYTES);
 #pragma unroll
                         for (int ks = 0; ks < 4; ks++) {
                             const uint64_t o = (uint64_t)ks * kstep;
-                            if (sizeof(T) == 4) umma_tf32(d, a + o, b + o, idesc, (kb > kb_begin || ks > 0) ? 1u : 0u);
-                            else umma_f16(d, a + o, b + o, idesc, (kb > kb_begin || ks > 0) ? 1u : 0u);
+                            if (sizeof(T) == 4) umma_tf32(d, a_hi + o, b_hi + o, idesc, ks > 0 ? 1u : first);
+                            else umma_f16(d, a_hi + o, b_hi + o, idesc, ks > 0 ? 1u : first);
                         }
                     }
                     umma_commit(&ctl->empty[s]);   // frees the stage once these MMAs have read it
+                    if (kb + 1 == kb_end) umma_commit(&ctl->tmem_full[ab]);
                 }
-                if (!dead) umma_commit(&ctl->tmem_full[ab]);
+                __syncwarp();
             }
-            if (p.debug && blockIdx.x == 0) { p.debug[1] = waited; p.debug[2] = waited2; }
         }
+        if (p.debug && blockIdx.x == 0 && lane == 0) { p.debug[1] = waited; p.debug[2] = waited2; }
     } else if (split_id >= 0) {
         // ------------------------------------------------------------ splitters (fp32 only)
         // Write, for every raw fp32 operand value the producers or TMA put into shared memory, the exact
@@ -776,12 +783,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         }
     } else if (warp == TMA_WARP ? tma_roles : (!tma_roles && warp >= 9)) {
         // ------------------------------------------------------------ producers
-        // TMA-fed launches: one lane of the TMA warp issues the copies.  Otherwise warps 9-16 gather with
+        // TMA-fed launches: the TMA warp runs as one, an elected lane issues the copies.  Otherwise warps 9-16 gather with
         // asynchronous 16-byte copies (zero-filled outside the image) straight into the swizzled
         // stage buffers, several stages ahead of the MMA.  Eight consecutive threads copy the
         // eight 16-byte chunks of one operand row, so a warp instruction reads four full 128-byte
         // lines; each thread serves rows (t/8), (t/8)+16, ... of the tile with its fixed chunk t%8.
-        const int pt = tma_roles ? lane : (warp - 9) * 32 + lane;   // gather: 0..255; TMA: lane 0 issues
+        const int pt = tma_roles ? lane : (warp - 9) * 32 + lane;   // gather: 0..255
         const T* __restrict__ X0 = reinterpret_cast<const T*>(p.x);
         const T* __restrict__ W0 = reinterpret_cast<const T*>(p.w);
         const bool vec = (p.C % C::EPC) == 0;
@@ -806,7 +813,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 // Filter gradient fed by TMA (float32).  A k-block is 32 consecutive output pixels; both operands
                 // stay pixel-major: four boxes of 32 pixels x 32 output channels of dy, and BN/32 im2col boxes of
                 // 32 pixels x 32 input channels of the layer input at this tile's tap.
-                if (pt == 0 && sizeof(T) == 4) {
+                if (sizeof(T) == 4) {
                     const bool multi = p.wg_tpt > 1;
                     const int tap0 = multi ? tn * p.wg_tpt : tn / p.ctiles;
                     const int cbase = multi ? 0 : (tn - tap0 * p.ctiles) * BN;
@@ -846,21 +853,24 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                             oq -= p.Q;
                             if (++op == p.P) { op = 0; n_img++; }
                         }
-                        if (!timed_wait(&ctl->empty[s], (ring.ph ^ 1u), abort_flag, waited)) {
+                        if (!timed_wait_warp(&ctl->empty[s], (ring.ph ^ 1u), abort_flag, waited)) {
                             if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_EMPTY); }
                             dead = true;
                             break;
                         }
                         const uint32_t a_dst = smem_u32(smem + s * stage_bytes);
                         const uint32_t b_dst = a_dst + b_off;
-                        mbar_arrive_expect_tx(&ctl->raw_full[s], C::A_BYTES + nb_boxes * 4096);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(&ctl->raw_full[s], C::A_BYTES + nb_boxes * 4096);
 #pragma unroll
-                        for (int g = 0; g < BM / 32; g++) tma_load_tile_2d(a_dst + g * 4096, p.tmap_a, &ctl->raw_full[s], k0 + 32 * g, (int)m0);
+                            for (int g = 0; g < BM / 32; g++) tma_load_tile_2d(a_dst + g * 4096, p.tmap_a, &ctl->raw_full[s], k0 + 32 * g, (int)m0);
 #pragma unroll
-                        for (int g = 0; g < BN / 32; g++)
-                            if (bc[g] >= 0)   // columns past C or past the last tap are never stored
-                                tma_load_im2col_4d(b_dst + g * 4096, p.tmap_b, &ctl->raw_full[s], bc[g], cur_q * p.stride_w - p.pad_w,
-                                                   cur_p * p.stride_h - p.pad_h, cur_n, boff_w[g], boff_h[g]);
+                            for (int g = 0; g < BN / 32; g++)
+                                if (bc[g] >= 0)   // columns past C or past the last tap are never stored
+                                    tma_load_im2col_4d(b_dst + g * 4096, p.tmap_b, &ctl->raw_full[s], bc[g], cur_q * p.stride_w - p.pad_w,
+                                                       cur_p * p.stride_h - p.pad_h, cur_n, boff_w[g], boff_h[g]);
+                        }
+                        __syncwarp();
                     }
                 } else {
                     break;
@@ -868,11 +878,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 continue;
             }
             if (p.use_tma) {
-                // Both operand tiles of a k-block arrive by one TMA copy each, issued by a single thread:
+                // Both operand tiles of a k-block arrive by one TMA copy each, issued by one elected lane:
                 // 128 im2col rows of the activation (zero outside the image, walking pixels in GEMM row
                 // order from the tile's first pixel) and BN filter rows, both landing in the 128-byte
                 // swizzled layout the MMA descriptors expect.
-                if (pt == 0) {
+                {
                     const long long m0 = (long long)tm * BM;
                     const int pq = p.OH * p.OW;
                     const int n_img = (int)(m0 / pq);
@@ -893,19 +903,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                         tc += C::BK;                       // next k-block: whole taps per k-block row (C % BK == 0), or one tap
                         if (tc >= p.C) { tc -= p.C; ts++; }
                         if (++kb_in_r == p.kblocks_per_r) { kb_in_r = 0; r++; ts = 0; tc = 0; }
-                        if (!timed_wait(&ctl->empty[s], (ring.ph ^ 1u), abort_flag, waited)) {
+                        if (!timed_wait_warp(&ctl->empty[s], (ring.ph ^ 1u), abort_flag, waited)) {
                             if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_EMPTY); }
                             dead = true;
                             break;
                         }
                         const uint32_t a_dst = smem_u32(smem + s * stage_bytes);
                         const uint32_t b_dst = a_dst + b_off;
-                        mbar_arrive_expect_tx(&ctl->raw_full[s], C::A_BYTES + C::B_BYTES);
-                        tma_load_im2col_4d(a_dst, p.tmap_a, &ctl->raw_full[s], cur_tc, cw, ch, cn, (uint16_t)off_w, (uint16_t)off_h);
-                        tma_load_tile_5d(b_dst, p.tmap_b, &ctl->raw_full[s], cur_tc, cur_ts, cur_r, tn * BN, bidx);
+                        if (elect_one()) {
+                            mbar_arrive_expect_tx(&ctl->raw_full[s], C::A_BYTES + C::B_BYTES);
+                            tma_load_im2col_4d(a_dst, p.tmap_a, &ctl->raw_full[s], cur_tc, cw, ch, cn, (uint16_t)off_w, (uint16_t)off_h);
+                            tma_load_tile_5d(b_dst, p.tmap_b, &ctl->raw_full[s], cur_tc, cur_ts, cur_r, tn * BN, bidx);
+                        }
+                        __syncwarp();
                     }
-                } else {
-                    break;   // the other producer threads have nothing to do
                 }
                 continue;
             }

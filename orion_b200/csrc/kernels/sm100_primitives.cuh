@@ -23,6 +23,18 @@ enum : int {
 // ~0.25 s at 1.9 GHz: far above any legitimate wait inside one kernel.
 #define OB200_WAIT_CYCLES (500ll * 1000 * 1000)
 
+// One lane of a converged warp.  MMAs and TMA copies are issued behind it by loops that the WHOLE warp runs, warp index taken
+// by shuffle: the compiler then knows descriptors, addresses and predicates to be the same for all lanes and keeps them in
+// uniform registers, where the instruction wants them.  Issued from a lane-0 branch each operand is moved there first: measured
+// 45 cycles per tcgen05.mma without and 65 - 100 with per-instruction selects, against 16 / 32 / 64 of the tensor core's own
+// for N = 32 / 64 / 128.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ int uniform_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -67,6 +79,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
         if (*abort_flag) return false;
         if (clock64() - t0 > OB200_WAIT_CYCLES) return false;
     }
+}
+
+// The same for a whole converged warp: every lane gets the same answer, so that a wait which runs out unwinds the warp as one.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
 }
 
 // One arrival that also announces `bytes` of asynchronous (TMA) transfers to come; the phase
