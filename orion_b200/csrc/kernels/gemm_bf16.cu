@@ -10,7 +10,11 @@
 // which the reference replays as cublasSgemm / cublasSgemmStridedBatched with transpose flags
 // (reference src/scheduler/utils_sched.cpp:490-513; rows of benchmarking/model_kernels/bert_8_fb1).
 //
-// One CTA = 128 x BN output tile per work unit, persistent over units.  Warp 0 issues TMA copies (4-D tensor maps:
+// One CTA = 128 x BN output tile per work unit, persistent over units; or a pair of CTAs (a cluster on the two SMs of a TPC,
+// cta_group::2) = 256 x BN, each CTA staging its 128 rows of A and half of B, so that an SM takes 32 KB instead of 48 KB of
+// operands from L2 per 128 x 256 x 64 product of its own.  Operand traffic is what bounds the single CTA (about 64 bytes a clock
+// and SM): decoder feed-forward 8192 x 4096 x 1024 56.6 -> 50.2 us (1.37 PFLOP/s), vocabulary projection 8192 x 32000 x 1024
+// 487 -> 411 us.  Warp 0 issues TMA copies (4-D tensor maps:
 // inner, outer, batch_inner, batch_outer; out-of-range elements read as zero, so ragged M, N, K need no special path),
 // warp 1 issues tcgen05.mma kind::f16 into one of two tensor-memory accumulators, warps 2-5 drain the other one:
 // tcgen05.ld (one output row per thread), alpha / bias / residual in registers, 32 rows x 128 bytes staged in a swizzled
@@ -40,10 +44,11 @@ constexpr int GM_BK = 64;
 constexpr int GM_THREADS = 192;          // warp 0: TMA, warp 1: MMA + tensor memory, warps 2-5: epilogue
 constexpr int GM_A_BYTES = GM_BM * 128;
 
-template <int BN>
+// CG CTAs (1, or a pair) share a tile of CG * 128 rows: each stages its 128 rows of A and BN / CG rows of B.
+template <int BN, int CG>
 struct GemmCfg {
-    static constexpr int STAGE_BYTES = GM_A_BYTES + BN * 128;
-    static constexpr int STAGES = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+    static constexpr int STAGE_BYTES = GM_A_BYTES + BN / CG * 128;
+    static constexpr int STAGES = STAGE_BYTES == 49152 ? 4 : STAGE_BYTES == 32768 ? 6 : 8;
     static constexpr int EPI_BYTES = 4 * 2 * 4096;   // per epilogue warp two slabs of 32 rows x 128 bytes for the TMA stores
     static constexpr int SMEM = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 256;
     static constexpr int TMEM_COLS = 2 * BN < 32 ? 32 : 2 * BN;
@@ -106,14 +111,15 @@ __device__ __forceinline__ bool gm_tile_skipped(const GemmParams& p, int tm, int
     return p.tri == 1 && tn * BN > tm * GM_BM + GM_BM - 1;
 }
 
-template <int BN>
+template <int BN, int CG>
 __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_constant__ GemmParams p) {
-    using C = GemmCfg<BN>;
+    using C = GemmCfg<BN, CG>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* epi_smem = smem + C::STAGES * C::STAGE_BYTES;
     GemmCtl* ctl = reinterpret_cast<GemmCtl*>(epi_smem + C::EPI_BYTES);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = uniform_warp_index(), lane = tid & 31;
+    const uint32_t rank = CG == 2 ? cluster_ctarank() : 0;   // CTA of the pair; CTA 0 issues the MMAs of both
 
     if (tid == 0) {
         for (int s = 0; s < C::STAGES; s++) {
@@ -122,7 +128,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(&ctl->acc_full[a], 1);
-            mbar_init(&ctl->acc_empty[a], 4);
+            mbar_init(&ctl->acc_empty[a], 4 * CG);   // the epilogue warps of both CTAs
         }
         ctl->abort_flag = 0;
         fence_barrier_init();
@@ -133,11 +139,17 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
         if (p.c_tma) prefetch_tensormap(p.tmap_c);
     }
     if (warp == 1) {
-        tmem_alloc(&ctl->tmem_base, C::TMEM_COLS);
-        tmem_relinquish();
+        if (CG == 2) {
+            tmem_alloc_pair(&ctl->tmem_base, C::TMEM_COLS);
+            tmem_relinquish_pair();
+        } else {
+            tmem_alloc(&ctl->tmem_base, C::TMEM_COLS);
+            tmem_relinquish();
+        }
         tc_fence_before_sync();
     }
     __syncthreads();
+    if (CG == 2) cluster_sync_all();   // the other CTA's barriers and tensor memory are ready
     tc_fence_after_sync();
     pdl_wait();
     if (tid == 0) pdl_launch_dependents();
@@ -147,56 +159,71 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
     const long long units = (long long)p.batch * tiles_per_problem * p.splits;
 
     if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            int s = 0;
-            uint32_t ph = 0;
-            bool dead = false;
-            for (long long u = blockIdx.x; u < units && !dead; u += gridDim.x) {
-                const int sp = (int)(u % p.splits);
-                const int tile = (int)(u / p.splits);
-                const int b = tile / tiles_per_problem, t = gm_rotate(p, tile - b * tiles_per_problem, b, tiles_per_problem);
-                const int tm = t / p.tiles_n, tn = t - tm * p.tiles_n;
-                const int bi = b % p.nb_inner, bo = b / p.nb_inner;
-                if (gm_tile_skipped<BN>(p, tm, tn)) continue;
-                int kb0, kb1;
-                gm_kb_range(p, sp, tm, kb0, kb1);
-                for (int kb = kb0; kb < kb1; kb++) {
-                    if (!mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag)) {
-                        if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_EMPTY); }
-                        dead = true;
-                        break;
-                    }
+        // ------------------------------------------------------------ TMA producer (the warp as one, see elect_one)
+        int s = 0;
+        uint32_t ph = 0;
+        bool dead = false;
+        for (long long u = blockIdx.x / CG; u < units && !dead; u += gridDim.x / CG) {
+            const int sp = (int)(u % p.splits);
+            const int tile = (int)(u / p.splits);
+            const int b = tile / tiles_per_problem, t = gm_rotate(p, tile - b * tiles_per_problem, b, tiles_per_problem);
+            const int tm = t / p.tiles_n, tn = t - tm * p.tiles_n;
+            const int bi = b % p.nb_inner, bo = b / p.nb_inner;
+            if (gm_tile_skipped<BN>(p, tm, tn)) continue;
+            int kb0, kb1;
+            gm_kb_range(p, sp, tm, kb0, kb1);
+            const int m0 = (tm * CG + (int)rank) * GM_BM, nb0 = tn * BN + (int)rank * (BN / CG);
+            for (int kb = kb0; kb < kb1; kb++) {
+                if (!mbar_wait_warp(&ctl->empty[s], ph ^ 1u, abort_flag)) {
+                    if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_EMPTY); }
+                    dead = true;
+                    break;
+                }
+                if (elect_one()) {
                     const uint32_t a_dst = smem_u32(smem + s * C::STAGE_BYTES);
                     const uint32_t b_dst = a_dst + GM_A_BYTES;
-                    mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)C::STAGE_BYTES);
+                    // the leading CTA's barrier counts the bytes of both CTAs
+                    if (rank == 0) mbar_arrive_expect_tx(&ctl->full[s], (uint32_t)(CG * C::STAGE_BYTES));
+                    const uint32_t bar = CG == 2 ? cluster_addr(smem_u32(&ctl->full[s]), 0) : 0;
+                    auto load = [&](uint32_t dst, const void* map, int c0, int c1) {
+                        if (CG == 2) tma_load_tile_4d_pair(dst, map, bar, c0, c1, bi, bo);
+                        else tma_load_tile_4d(dst, map, &ctl->full[s], c0, c1, bi, bo);
+                    };
                     if (!p.a_mn) {
-                        tma_load_tile_4d(a_dst, p.tmap_a, &ctl->full[s], kb * GM_BK, tm * GM_BM, bi, bo);
+                        load(a_dst, p.tmap_a, kb * GM_BK, m0);
                     } else {
 #pragma unroll
-                        for (int g = 0; g < GM_BM / 64; g++)
-                            tma_load_tile_4d(a_dst + g * 8192, p.tmap_a, &ctl->full[s], tm * GM_BM + 64 * g, kb * GM_BK, bi, bo);
+                        for (int g = 0; g < GM_BM / 64; g++) load(a_dst + g * 8192, p.tmap_a, m0 + 64 * g, kb * GM_BK);
                     }
                     if (!p.b_mn) {
-                        tma_load_tile_4d(b_dst, p.tmap_b, &ctl->full[s], kb * GM_BK, tn * BN, bi, bo);
+                        load(b_dst, p.tmap_b, kb * GM_BK, nb0);
                     } else {
 #pragma unroll
-                        for (int g = 0; g < BN / 64; g++)
-                            tma_load_tile_4d(b_dst + g * 8192, p.tmap_b, &ctl->full[s], tn * BN + 64 * g, kb * GM_BK, bi, bo);
+                        for (int g = 0; g < BN / CG / 64; g++) load(b_dst + g * 8192, p.tmap_b, nb0 + 64 * g, kb * GM_BK);
                     }
-                    if (++s == C::STAGES) { s = 0; ph ^= 1u; }
                 }
+                __syncwarp();
+                if (++s == C::STAGES) { s = 0; ph ^= 1u; }
             }
         }
+        // The leading CTA's commits arrive on this CTA's barriers: they must have landed before either CTA leaves.
+        for (int i = 0; CG == 2 && i < C::STAGES && !dead; i++) {
+            if (!mbar_wait_warp(&ctl->empty[s], ph ^ 1u, abort_flag)) break;
+            if (++s == C::STAGES) { s = 0; ph ^= 1u; }
+        }
     } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issue
-        if (lane == 0) {
-            const uint32_t idesc = umma_idesc(1, GM_BM, BN) | (p.a_mn ? UMMA_IDESC_A_MN : 0u) | (p.b_mn ? UMMA_IDESC_B_MN : 0u);
+        // ------------------------------------------------------------ MMA issue (the warp as one)
+        if (rank == 0) {
+            const uint32_t idesc = umma_idesc(1, CG * GM_BM, BN) | (p.a_mn ? UMMA_IDESC_A_MN : 0u) | (p.b_mn ? UMMA_IDESC_B_MN : 0u);
+            // descriptors above the address; 16 reduction indices further on: 32 bytes along a K-major row, two 8-row atoms of
+            // an MN-major tile
+            const uint64_t a_bits = p.a_mn ? gm_desc_mn(0) : umma_desc_sw128(0), b_bits = p.b_mn ? gm_desc_mn(0) : umma_desc_sw128(0);
+            const uint64_t a_step = p.a_mn ? 2048 >> 4 : 2, b_step = p.b_mn ? 2048 >> 4 : 2;
             int s = 0;
             uint32_t ph = 0;
             uint32_t local = 0;
             bool dead = false;
-            for (long long u = blockIdx.x; u < units && !dead; u += gridDim.x) {
+            for (long long u = blockIdx.x / CG; u < units && !dead; u += gridDim.x / CG) {
                 const int sp = (int)(u % p.splits);
                 const int tile = (int)(u / p.splits);
                 const int t = gm_rotate(p, tile % tiles_per_problem, tile / tiles_per_problem, tiles_per_problem);
@@ -206,31 +233,38 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
                 gm_kb_range(p, sp, tm, kb0, kb1);
                 const uint32_t ab = local & 1u, use = local >> 1;
                 local++;
-                if (!mbar_wait(&ctl->acc_empty[ab], (use & 1u) ^ 1u, abort_flag)) {
+                if (!mbar_wait_warp(&ctl->acc_empty[ab], (use & 1u) ^ 1u, abort_flag)) {
                     if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_EMPTY); }
                     break;
                 }
                 tc_fence_after_sync();
                 const uint32_t d = tmem_base + ab * BN;
                 for (int kb = kb0; kb < kb1; kb++) {
-                    if (!mbar_wait(&ctl->full[s], ph, abort_flag)) {
+                    if (!mbar_wait_warp(&ctl->full[s], ph, abort_flag)) {
                         if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
                         dead = true;
                         break;
                     }
                     tc_fence_after_sync();
-                    const uint32_t a_base = smem_u32(smem + s * C::STAGE_BYTES), b_base = a_base + GM_A_BYTES;
+                    const uint32_t first = kb > kb0 ? 1u : 0u;   // 0: the tile's first product overwrites the accumulator
+                    if (elect_one()) {
+                        const uint32_t a_base = smem_u32(smem + s * C::STAGE_BYTES);
+                        const uint64_t ad = umma_desc_mn(a_bits, a_base), bd = umma_desc_mn(b_bits, a_base + GM_A_BYTES);
 #pragma unroll
-                    for (int ks = 0; ks < GM_BK / 16; ks++) {
-                        // 16 reduction indices further on: 32 bytes along a K-major row, two 8-row atoms of an MN-major tile
-                        const uint64_t ad = p.a_mn ? gm_desc_mn(a_base + ks * 2048) : umma_desc_sw128(a_base) + (uint64_t)ks * 2;
-                        const uint64_t bd = p.b_mn ? gm_desc_mn(b_base + ks * 2048) : umma_desc_sw128(b_base) + (uint64_t)ks * 2;
-                        umma_f16(d, ad, bd, idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 0; ks < GM_BK / 16; ks++) {
+                            if (CG == 2) umma_f16_pair(d, ad + ks * a_step, bd + ks * b_step, idesc, ks > 0 ? 1u : first);
+                            else umma_f16(d, ad + ks * a_step, bd + ks * b_step, idesc, ks > 0 ? 1u : first);
+                        }
+                        if (CG == 2) umma_commit_pair(&ctl->empty[s]);
+                        else umma_commit(&ctl->empty[s]);
+                        if (kb + 1 == kb1) {
+                            if (CG == 2) umma_commit_pair(&ctl->acc_full[ab]);
+                            else umma_commit(&ctl->acc_full[ab]);
+                        }
                     }
-                    umma_commit(&ctl->empty[s]);
+                    __syncwarp();
                     if (++s == C::STAGES) { s = 0; ph ^= 1u; }
                 }
-                if (!dead) umma_commit(&ctl->acc_full[ab]);
             }
         }
     } else {
@@ -239,7 +273,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
         const int r = q * 32 + lane;
         uint32_t local = 0;
         uint32_t slab_i = 0;
-        for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        for (long long u = blockIdx.x / CG; u < units; u += gridDim.x / CG) {
             const int sp = (int)(u % p.splits);
             const int tile = (int)(u / p.splits);
             const int b = tile / tiles_per_problem, t = gm_rotate(p, tile - b * tiles_per_problem, b, tiles_per_problem);
@@ -253,7 +287,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
                 break;
             }
             tc_fence_after_sync();
-            const int m = tm * GM_BM + r;
+            const int m = (tm * CG + (int)rank) * GM_BM + r;
             const int n0 = tn * BN;
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + ab * BN;
             const bool to_slab = p.splits > 1;
@@ -261,7 +295,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
             float* srow = to_slab ? p.slabs + (((long long)sp * p.batch + b) * p.M + m) * p.N : nullptr;
             const long long c_off = (long long)bo * p.c_so + (long long)bi * p.c_si + (long long)m * p.ldc;
             const bool by_tma = p.c_tma && !to_slab;
-            const int m0w = tm * GM_BM + q * 32;      // first row of this warp's 32
+            const int m0w = (tm * CG + (int)rank) * GM_BM + q * 32;      // first row of this warp's 32
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 32) {
                 if (n0 + c0 >= p.N) break;            // warp-uniform
@@ -390,14 +424,21 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&ctl->acc_empty[ab]);
+            if (lane == 0) {
+                if (CG == 2) mbar_arrive_cluster(cluster_addr(smem_u32(&ctl->acc_empty[ab]), 0));
+                else mbar_arrive(&ctl->acc_empty[ab]);
+            }
         }
         if (lane == 0) bulk_wait_group<0>();   // the slabs must outlive the stores that read them
     }
+    tc_fence_before_sync();
     __syncthreads();
+    if (CG == 2) cluster_sync_all();   // nothing of this CTA is used by the other one any more
     if (warp == 1) {
+        __syncwarp();
         tc_fence_after_sync();
-        tmem_dealloc(tmem_base, C::TMEM_COLS);
+        if (CG == 2) tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
+        else tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
 }
 
@@ -453,35 +494,46 @@ static bool gm_make_map(unsigned char* out, const void* base, long long inner, l
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
+template <int BN, int CG>
 static int gm_launch(const GemmParams& p, int grid, cudaStream_t stream) {
     static bool attr_set[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 64 && !attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<BN, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN, CG>::SMEM);
         if (e != cudaSuccess) return (int)e;
         attr_set[dev] = true;
     }
-    OB200_ELASTIC(gemm_bf16_kernel<BN>, 1);
+    OB200_ELASTIC((gemm_bf16_kernel<BN, CG>), 1);
     // Programmatic dependent launch: the kernel's set-up (barriers, tensor memory, descriptor prefetch) may overlap the tail of
     // the kernel before it in the stream; it reads and writes global memory only behind its griddepcontrol.wait.
     static const bool pdl = [] {   // ORION_PDL=0: plain stream order between consecutive kernels
         const char* e = getenv("ORION_PDL");
         return !(e && e[0] == '0');
     }();
+    if (CG == 2) grid = grid < 2 ? 2 : grid & ~1;   // whole pairs
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(GM_THREADS);
-    cfg.dynamicSmemBytes = GemmCfg<BN>::SMEM;
+    cfg.dynamicSmemBytes = GemmCfg<BN, CG>::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (CG == 2) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 2;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        n++;
+    }
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n].val.programmaticStreamSerializationAllowed = 1;
+        n++;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<BN>, p);
+    cfg.numAttrs = (unsigned)n;
+    return (int)cudaLaunchKernelEx(&cfg, gemm_bf16_kernel<BN, CG>, p);
 }
 
 }  // namespace ob200
@@ -532,28 +584,38 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
     const int cal = out_f32 ? 4 : 8;   // elements per 16 bytes of C
     p.vec_ok = ((uintptr_t)c % 16 == 0) && ((uintptr_t)residual % 16 == 0) && (!residual || !out_f32) && (ldc % cal == 0) && (batch_inner == 1 || c_si % cal == 0) && (batch_outer == 1 || c_so % cal == 0);
     const int plan = ob200_plan_sm_count();
-    const int tiles_m = (M + GM_BM - 1) / GM_BM;
-    // Tile width: 256 columns halve the re-reads of A where the grid still fills the device; 64 for narrow outputs.
-    // A 128 x 128 tile is bound by operand traffic (32 KB per k-block), a 128 x 256 tile takes about 1.5 times as long for
-    // twice the work: pick the width whose number of waves times that cost is smaller.
-    int bn = N <= 64 ? 64 : 128;
-    if (N >= 256) {
-        const long long t128 = batch_ll * tiles_m * ((N + 127) / 128), t256 = batch_ll * tiles_m * ((N + 255) / 256);
-        const long long w128 = (t128 + plan - 1) / plan, w256 = (t256 + plan - 1) / plan;
-        if (w256 * 3 < w128 * 2 + 1 && t256 * 2 > plan) bn = 256;
-    }
-    p.tiles_m = tiles_m;
-    p.tiles_n = (N + bn - 1) / bn;
     p.kblocks = (K + GM_BK - 1) / GM_BK;
+    // Tile and split: the smallest modelled time, in hundredths of what a 128 x 128 tile takes for a k-block (0.33 us).  Measured
+    // over 8192 x 4096 x 1024 and 8192 x 32000 x 1024 (us per wave of tiles): 5.3 / 5.6 for 128 x 128, 8.1 / 8.9 for 128 x 256,
+    // 4.6 / 4.9 for a pair's 256 x 128, 7.2 / 7.5 for its 256 x 256: what tells them apart is the operand bytes that an SM takes
+    // from L2 per k-block (32, 48, 24, 32 KB).  Split-K (few tiles, long reduction) adds writing and reading its partial matrices
+    // at about 6 TB/s.  Planned for the device's SM count, never for the quota of the call, so the summation order (and the
+    // result, bit for bit) is the same for every quota.
+    struct Tile { int bn, cg, cost; };
+    static const Tile kTiles[] = {{128, 1, 100}, {256, 1, 155}, {128, 2, 88}, {256, 2, 136}};
+    static const Tile kNarrow[] = {{64, 1, 100}};   // outputs of at most 64 columns
+    int bn = 64, cg = 1, splits = 1;
+    double best = -1.0;
+    for (const Tile& t : kTiles) {
+        const Tile& c = N <= 64 ? kNarrow[0] : t;
+        if ((c.bn == 256 && N < 256) || (c.cg == 2 && (M <= GM_BM || tri != 0))) continue;
+        const long long tiles = batch_ll * ((M + c.cg * GM_BM - 1) / (c.cg * GM_BM)) * ((N + c.bn - 1) / c.bn);
+        const long long at_once = plan / c.cg > 0 ? plan / c.cg : 1;
+        int sp = 1;
+        if (tiles * 2 <= at_once && p.kblocks >= 8 && tri == 0) {
+            sp = (int)(at_once / tiles);
+            if (sp > p.kblocks / 4) sp = p.kblocks / 4;
+            if (sp > 16) sp = 16;
+        }
+        const double waves = (double)((tiles * sp + at_once - 1) / at_once);
+        const double cost = waves * c.cost * ((p.kblocks + sp - 1) / sp) + (sp > 1 ? (double)sp * batch_ll * M * N / 2500.0 : 0.0);
+        if (best < 0.0 || cost < best) { best = cost; bn = c.bn; cg = c.cg; splits = sp; }
+    }
+    p.tiles_m = (M + cg * GM_BM - 1) / (cg * GM_BM);
+    p.tiles_n = (N + bn - 1) / bn;
     const long long tiles = batch_ll * p.tiles_m * p.tiles_n;
     if (tiles > 0x7fffffffLL) return -1;
-    // Split-K: few tiles, long reduction.  Planned for the device's SM count, never for the quota of the call, so the
-    // summation order (and the result, bit for bit) is the same for every quota.
-    int splits = 1;
-    if (tiles * 2 <= plan && p.kblocks >= 8 && tri == 0) {
-        splits = (int)(plan / tiles);
-        if (splits > p.kblocks / 4) splits = p.kblocks / 4;
-        if (splits > 16) splits = 16;
+    if (splits > 1) {
         size_t slab_bytes = 0;
         float* slabs = ob200_stream_slabs(stream, &slab_bytes);
         const size_t per_split = (size_t)batch_ll * M * N * sizeof(float);
@@ -568,7 +630,7 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
     const bool ok_a = a_mn ? gm_make_map(p.tmap_a, a, M, K, lda, batch_inner, a_si, batch_outer, a_so, 64, GM_BK)
                            : gm_make_map(p.tmap_a, a, K, M, lda, batch_inner, a_si, batch_outer, a_so, GM_BK, GM_BM);
     const bool ok_b = b_mn ? gm_make_map(p.tmap_b, b, N, K, ldb, batch_inner, b_si, batch_outer, b_so, 64, GM_BK)
-                           : gm_make_map(p.tmap_b, b, K, N, ldb, batch_inner, b_si, batch_outer, b_so, GM_BK, bn);
+                           : gm_make_map(p.tmap_b, b, K, N, ldb, batch_inner, b_si, batch_outer, b_so, GM_BK, bn / cg);
     if (!ok_a || !ok_b) return -4;
     // C by TMA stores when its rows and batch offsets are 16-byte multiples (always true for the layouts of the clients)
     {
@@ -590,13 +652,13 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
         }
     }
     const long long units = tiles * p.splits;
-    int grid = units < num_ctas ? (int)units : num_ctas;
+    int grid = units * cg < num_ctas ? (int)(units * cg) : num_ctas;
     // ORION_GEMM_TILES_PER_CTA=t (t > 0): a CTA retires after about t work units instead of staying for the whole launch, so
     // that the blocks of a higher-priority kernel find a free SM after a few microseconds (the grid is then wider than the
     // quota; the scheduler's cut to the quota, where it applies, still holds).
     static const int tiles_per_cta = [] { const char* e = getenv("ORION_GEMM_TILES_PER_CTA"); return e ? atoi(e) : 0; }();
     if (tiles_per_cta > 0) {
-        const long long want = (units + tiles_per_cta - 1) / tiles_per_cta;
+        const long long want = (units + tiles_per_cta - 1) / tiles_per_cta * cg;
         if (want > grid) grid = want > 0x7fffffffLL ? 0x7fffffff : (int)want;
     }
     {
@@ -604,8 +666,9 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
         const double bytes = 2.0 * batch_ll * ((double)M * K + (double)N * K) + (out_f32 ? 4.0 : 2.0) * batch_ll * (double)M * N;
         annotate_launch(flop / bytes > ai_threshold(1) ? 1 : 0, flop, bytes);
     }
-    int rc = bn == 256 ? gm_launch<256>(p, grid, (cudaStream_t)stream)
-                       : bn == 128 ? gm_launch<128>(p, grid, (cudaStream_t)stream) : gm_launch<64>(p, grid, (cudaStream_t)stream);
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc = cg == 2 ? (bn == 256 ? gm_launch<256, 2>(p, grid, st) : gm_launch<128, 2>(p, grid, st))
+             : bn == 256 ? gm_launch<256, 1>(p, grid, st) : bn == 128 ? gm_launch<128, 1>(p, grid, st) : gm_launch<64, 1>(p, grid, st);
     if (rc != 0 || p.splits == 1) return rc;
     const long long elems = batch_ll * M * N;
     long long blocks = (elems + 255) / 256;

@@ -49,6 +49,26 @@ def test_bias_and_alpha(built):
     _check(c, _ref(a, b, False, False, bias, 0.125), 256)
 
 
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K", [(129, 128, 64), (257, 264, 72), (384, 136, 200), (2200, 2040, 136), (136, 72, 2056)])
+def test_tiles_of_cta_pairs_at_their_edges(built, trans_a, trans_b, M, N, K):
+    """256-row tiles shared by two CTAs (128 and 256 columns wide, with and without split-K): rows and columns past the edge in
+    one CTA or in both, and the same bits for an even, an odd and the smallest CTA count."""
+    from orion_b200 import kernels as K_
+    torch.manual_seed(M + N + K)
+    def mat(rows, cols):
+        ld = (cols + 7) // 8 * 8
+        return torch.randn(rows, ld, device="cuda").to(torch.bfloat16)[:, :cols]
+    a = mat(K, M) if trans_a else mat(M, K)
+    b = mat(K, N) if trans_b else mat(N, K)
+    ref = _ref(a, b, trans_a, trans_b, None, 1.0)
+    outs = [K_.gemm_bf16(a, b, trans_a, trans_b, out_dtype=torch.float32, num_ctas=n) for n in (148, 7, 1)]
+    _check(outs[0], ref, K)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    _check(K_.gemm_bf16(a, b, trans_a, trans_b), ref, K)
+    assert K_.read_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(768, 768, 3072), (2304, 768, 3072), (1024, 1024, 8192), (768, 136, 2000)])
 def test_weight_gradient_shapes_take_split_k_and_do_not_depend_on_the_cta_count(built, M, N, K):
     """dW = dY^T . X: both operands [tokens, features]; few output tiles and a long reduction."""
