@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(NT_THREADS) bias_gelu_backward_kernel(const T*
 #pragma unroll
                 for (int e = 0; e < N; e++) {
                     const float a = v[e] + b[e];
-                    const float ex = __expf(-0.5f * a * a);
+                    const float ex = gauss_exp(a);
                     const float cdf = gauss_cdf_with_exp(a, ex);
                     const float pdf = 0.3989422804014327f * ex;
                     d[e] *= cdf + a * pdf;
