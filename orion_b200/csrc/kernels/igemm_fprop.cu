@@ -79,8 +79,10 @@ struct Cfg {
     static constexpr int BY_TMEM = ATMEM ? (512 - 2 * BN) / 64 : 8;      // 64 tensor-memory columns per stage
     static constexpr int STAGES = BY_SMEM < BY_TMEM ? (BY_SMEM > 8 ? 8 : BY_SMEM) : (BY_TMEM > 8 ? 8 : BY_TMEM);
     static constexpr int RING_BYTES = STAGES * STAGE_BYTES;
-    static constexpr int EPI_BYTES = 2 * EPI_WARPS * 32 * 20 * 4;   // per-warp transpose tiles of the epilogue (EPI_LD floats per row)
+    // per epilogue warp: 32 rows x 128 bytes for TMA stores, or the transpose tile of the other path (EPI_LD floats per row)
+    static constexpr int EPI_BYTES = 2 * EPI_WARPS * 4096;
     static constexpr int SMEM_BYTES = RING_BYTES + EPI_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+    static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
     // Two accumulators of BN columns; ATMEM adds, per stage, the two parts of the activation tile (32 + 32 columns).
     // Allocations are powers of two.
     static constexpr int A_TMEM_COL0 = 2 * BN;
@@ -308,6 +310,43 @@ __device__ __forceinline__ void epilogue_chunk(const IgemmParams& p, float* stag
     __syncwarp();
 }
 
+// Epilogue of one 32-row x 32-column accumulator chunk held one row per lane, written by a TMA store: scale / shift (the same
+// address for all lanes), activation, eight 16-byte shared-memory stores of the lane's row in the 128-byte swizzle, one copy of
+// the 32 x 32 box, which clips rows past M and columns past Kout.  A third of the instructions of the transposing path above,
+// nearly all of them independent: a 128 x 128 tile took that path 10 000 cycles of eight warps (each a chain of latencies) and
+// bound every layer of up to 16 k-blocks.
+__device__ __forceinline__ void epilogue_store32(const IgemmParams& p, float* slab, float (&x)[32], int lane, long long row0, int n0) {
+    if (p.scale || p.shift) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 4) {
+            if (n0 + j >= p.Kout) break;   // Kout is a multiple of four
+            const float4 sc = p.scale ? __ldg(reinterpret_cast<const float4*>(p.scale + n0 + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
+            const float4 sh = p.shift ? __ldg(reinterpret_cast<const float4*>(p.shift + n0 + j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            x[j] = fmaf(x[j], sc.x, sh.x);
+            x[j + 1] = fmaf(x[j + 1], sc.y, sh.y);
+            x[j + 2] = fmaf(x[j + 2], sc.z, sh.z);
+            x[j + 3] = fmaf(x[j + 3], sc.w, sh.w);
+        }
+    }
+    if (p.relu) {
+        const float top = p.relu == 2 ? 6.f : INFINITY;
+#pragma unroll
+        for (int j = 0; j < 32; j++) x[j] = fminf(fmaxf(x[j], 0.f), top);
+    }
+    if (lane == 0) bulk_wait_group_read<0>();   // the copy issued from this slab before has read it
+    __syncwarp();
+    uint8_t* row = reinterpret_cast<uint8_t*>(slab) + lane * 128;
+#pragma unroll
+    for (int ch = 0; ch < 8; ch++)
+        *reinterpret_cast<float4*>(row + ((ch ^ (lane & 7)) << 4)) = make_float4(x[4 * ch], x[4 * ch + 1], x[4 * ch + 2], x[4 * ch + 3]);
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && row0 < p.M) {
+        tma_store_tile_2d(p.tmap_y, smem_u32(slab), n0, (int)row0);
+        bulk_commit_group();
+    }
+}
+
 // mbar_wait that also adds the cycles spent waiting to `acc` (role-level wait breakdown for tuning).
 __device__ __forceinline__ bool timed_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long& acc) {
     const long long t0 = clock64();   // the first try_wait may already suspend the thread for a while
@@ -431,6 +470,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
     if (warp == TMA_WARP && lane == 0 && p.use_tma) {
         prefetch_tensormap(p.tmap_a);   // hide the descriptor fetch behind the rest of the set-up
         prefetch_tensormap(p.tmap_b);
+        if (p.y_tma) prefetch_tensormap(p.tmap_y);
     }
     __syncthreads();   // barriers are initialised: the TMA warp may start copying
     // Everything above touched only this CTA's shared memory and the kernel parameters, so under programmatic
@@ -475,7 +515,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         const int grp = epi_id >> 2;
         const int col_lo = grp * (BN / epi_groups), col_hi = col_lo + BN / epi_groups;
         const int epi_threads = 128 * epi_groups;
-        float* stage = epi_stage + epi_id * (32 * EPI_LD);
+        float* stage = epi_stage + epi_id * 1024;
         const int sub = lane >> 2;          // row within a group of eight
         const int cc = (lane & 3) * 4;      // first of this lane's four channels within a 16-channel chunk
         const uint32_t tmem_rows = tmem_base + ((uint32_t)(q * 32) << 16);
@@ -586,6 +626,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 if (ctl->last_flag) {
                     // Last piece to arrive: every slab of the tile is published.  Sum them in CTA (split) order.
                     __threadfence();
+                    if (sizeof(T) == 4 && p.y_tma) {
+#pragma unroll 1
+                        for (int c32 = col_lo; c32 < col_hi && tn * BN + c32 < p.Kout; c32 += 32) {
+                            float acc[32];
+#pragma unroll
+                            for (int j = 0; j < 32; j++) acc[j] = 0.f;
+                            for (int c = seg.first_cta; c < seg.first_cta + seg.nseg; c++) {
+                                const float4* src = slabs + (long long)work.slab_of(c, tile) * SLAB_F4;
+#pragma unroll
+                                for (int j = 0; j < 8; j++) {
+                                    const float4 v = __ldcg(src + (c32 / 4 + j) * BM + row);
+                                    acc[4 * j] += v.x; acc[4 * j + 1] += v.y; acc[4 * j + 2] += v.z; acc[4 * j + 3] += v.w;
+                                }
+                            }
+                            epilogue_store32(p, stage, acc, lane, tile_row0, tn * BN + c32);
+                        }
+                    } else
 #pragma unroll 1
                     for (int c16 = col_lo; c16 < col_hi; c16 += 16) {
                         float acc[16];
@@ -608,8 +665,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             }
 #pragma unroll 1
             for (int c32 = col_lo; c32 < col_hi; c32 += 32) {   // whole tile in one piece: straight to the output
+                if (tn * BN + c32 >= p.Kout) break;
                 uint32_t r[32];
                 load_acc((uint32_t)(ab * BN + c32), r);
+                if (sizeof(T) == 4 && p.y_tma) {
+                    float x[32];
+#pragma unroll
+                    for (int j = 0; j < 32; j++) x[j] = __uint_as_float(r[j]);
+                    epilogue_store32(p, stage, x, lane, tile_row0, tn * BN + c32);
+                    continue;
+                }
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     float v16[16];
@@ -622,6 +687,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl->tmem_empty[ab]);
         }
+        if (lane == 0) bulk_wait_group<0>();   // the slabs must outlive the copies that read them
         if (p.debug && blockIdx.x == 0 && tid == 0) p.debug[0] = waited;
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------ MMA issue (the warp as one, see elect_one)
@@ -1299,6 +1365,23 @@ static bool setup_tma(IgemmParams& p, int bn) {
 
 }  // namespace ob200
 
+// float32 outputs whose rows are whole 16-byte groups, stored in place and without a residual, leave by TMA stores.
+static void setup_tma_store(IgemmParams& p) {
+    using namespace ob200;
+    p.y_tma = 0;
+    const TmaApi& api = tma_api();
+    if (!api.ok || p.mode != 0 || p.dtype == 1 || p.out_map || p.batch > 1 || p.residual || (p.Kout & 3)) return;
+    if (((uintptr_t)p.y | (uintptr_t)p.scale | (uintptr_t)p.shift) % 16) return;
+    cuuint64_t dims[2] = {(cuuint64_t)p.Kout, (cuuint64_t)p.M};
+    cuuint64_t strides[1] = {(cuuint64_t)p.Kout * 4};
+    cuuint32_t box[2] = {32, 32};
+    cuuint32_t steps[2] = {1, 1};
+    if (api.tiled(reinterpret_cast<CUtensorMap*>(p.tmap_y), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.y, dims, strides, box, steps,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+        p.y_tma = 1;
+}
+
 static std::atomic<long long> g_tma_launches{0};
 
 extern "C" long long ob200_tma_launch_count(void) { return g_tma_launches.load(std::memory_order_relaxed); }
@@ -1329,6 +1412,7 @@ extern "C" int ob200_igemm_launch(const IgemmParams* params, int bn, int num_cta
     }
     if (setup_tma(p, bn)) g_tma_launches.fetch_add(1, std::memory_order_relaxed);
     else if (p.require_tma || p.w_R > 0) return -4;   // tap subsets exist only on the TMA path
+    setup_tma_store(p);
     {   // class of this launch for the scheduler's profiles: arithmetic intensity of the problem against the device's
         const double batch = p.batch > 1 ? p.batch : 1;
         const double elem = p.dtype == 1 ? 2.0 : 4.0;

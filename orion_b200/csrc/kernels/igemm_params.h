@@ -89,6 +89,8 @@ typedef struct IgemmParams {
     int cross_acc;
     int tma_base_h, tma_base_w;
     unsigned long long mn_desc_bits;   /* filter gradient on TMA: the operand descriptors' bits above the address */
+    int y_tma;         /* y is written by TMA stores (tmap_y: [M, Kout] in boxes of 32 x 32 float32) */
+    OB200_ALIGN64 unsigned char tmap_y[128];
     OB200_ALIGN64 unsigned char tmap_a[128];
     OB200_ALIGN64 unsigned char tmap_b[128];
 } IgemmParams;
