@@ -96,6 +96,7 @@ struct SharedCtl {
     uint64_t empty[8];
     uint64_t tmem_full[2];
     uint64_t tmem_empty[2];
+    uint64_t res_full[2 * EPI_WARPS];   // per epilogue warp: its residual box has landed
     uint32_t tmem_base;
     int abort_flag;
     int last_flag;
@@ -315,7 +316,19 @@ __device__ __forceinline__ void epilogue_chunk(const IgemmParams& p, float* stag
 // the 32 x 32 box, which clips rows past M and columns past Kout.  A third of the instructions of the transposing path above,
 // nearly all of them independent: a 128 x 128 tile took that path 10 000 cycles of eight warps (each a chain of latencies) and
 // bound every layer of up to 16 k-blocks.
-__device__ __forceinline__ void epilogue_store32(const IgemmParams& p, float* slab, float (&x)[32], int lane, long long row0, int n0) {
+// A residual arrives in the slab by a TMA copy issued ahead of the accumulator (fetch_residual32) and is added there in place.
+__device__ __forceinline__ void fetch_residual32(const IgemmParams& p, float* slab, uint64_t* bar, int lane, long long row0, int n0) {
+    if (lane == 0) {
+        bulk_wait_group_read<0>();   // the copy issued from this slab before has read it
+        mbar_arrive_expect_tx(bar, 4096);
+        tma_load_tile_2d(smem_u32(slab), p.tmap_r, bar, n0, (int)row0);
+    }
+    __syncwarp();
+}
+// False if the residual did not arrive.
+__device__ __forceinline__ bool epilogue_store32(const IgemmParams& p, float* slab, float (&x)[32], uint64_t* res_bar, uint32_t res_phase,
+                                                 volatile int* abort_flag, int lane, long long row0, int n0) {
+    uint8_t* row = reinterpret_cast<uint8_t*>(slab) + lane * 128;
     if (p.scale || p.shift) {
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
@@ -328,14 +341,22 @@ __device__ __forceinline__ void epilogue_store32(const IgemmParams& p, float* sl
             x[j + 3] = fmaf(x[j + 3], sc.w, sh.w);
         }
     }
+    if (p.residual) {
+        if (!mbar_wait_warp(res_bar, res_phase, abort_flag)) return false;
+#pragma unroll
+        for (int ch = 0; ch < 8; ch++) {
+            const float4 v = *reinterpret_cast<const float4*>(row + ((ch ^ (lane & 7)) << 4));
+            x[4 * ch] += v.x; x[4 * ch + 1] += v.y; x[4 * ch + 2] += v.z; x[4 * ch + 3] += v.w;
+        }
+    } else {
+        if (lane == 0) bulk_wait_group_read<0>();   // the copy issued from this slab before has read it
+        __syncwarp();
+    }
     if (p.relu) {
         const float top = p.relu == 2 ? 6.f : INFINITY;
 #pragma unroll
         for (int j = 0; j < 32; j++) x[j] = fminf(fmaxf(x[j], 0.f), top);
     }
-    if (lane == 0) bulk_wait_group_read<0>();   // the copy issued from this slab before has read it
-    __syncwarp();
-    uint8_t* row = reinterpret_cast<uint8_t*>(slab) + lane * 128;
 #pragma unroll
     for (int ch = 0; ch < 8; ch++)
         *reinterpret_cast<float4*>(row + ((ch ^ (lane & 7)) << 4)) = make_float4(x[4 * ch], x[4 * ch + 1], x[4 * ch + 2], x[4 * ch + 3]);
@@ -345,6 +366,7 @@ __device__ __forceinline__ void epilogue_store32(const IgemmParams& p, float* sl
         tma_store_tile_2d(p.tmap_y, smem_u32(slab), n0, (int)row0);
         bulk_commit_group();
     }
+    return true;
 }
 
 // mbar_wait that also adds the cycles spent waiting to `acc` (role-level wait breakdown for tuning).
@@ -463,6 +485,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             mbar_init(&ctl->tmem_full[b], 1);           // tcgen05.commit
             mbar_init(&ctl->tmem_empty[b], p.use_tma ? 2 * EPI_WARPS : EPI_WARPS);  // one elected lane per epilogue warp
         }
+        for (int w = 0; w < 2 * EPI_WARPS; w++) mbar_init(&ctl->res_full[w], 1);   // the lane that issues the copy, and its bytes
         ctl->abort_flag = 0;
         ctl->last_flag = 0;
         fence_barrier_init();
@@ -471,6 +494,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         prefetch_tensormap(p.tmap_a);   // hide the descriptor fetch behind the rest of the set-up
         prefetch_tensormap(p.tmap_b);
         if (p.y_tma) prefetch_tensormap(p.tmap_y);
+        if (p.y_tma && p.residual) prefetch_tensormap(p.tmap_r);
     }
     __syncthreads();   // barriers are initialised: the TMA warp may start copying
     // Everything above touched only this CTA's shared memory and the kernel parameters, so under programmatic
@@ -536,10 +560,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 tmem_ld_wait();
             }
         };
+        const bool fetch = sizeof(T) == 4 && p.y_tma && p.residual != nullptr;
+        uint64_t* res_bar = &ctl->res_full[epi_id];
+        uint32_t res_phase = 0;
+        bool res_ok = true;
         int local = 0;
         WorkIter work(p, tiles);
         Seg seg;
-        for (; work.next(seg); local++) {
+        for (; res_ok && work.next(seg); local++) {
             const int tile = seg.tile;
             const int bidx = tile / tiles_per_problem;
             const int tloc = tile - bidx * tiles_per_problem;
@@ -548,12 +576,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             // With the cross-term accumulator there is one output buffer (0) and its barriers flip every tile.
             const int ab = cross ? 0 : (local & 1);
             const uint32_t acc_use = cross ? (uint32_t)local : (uint32_t)(local >> 1);
-            if (!timed_wait(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
+            const long long tile_row0 = (long long)tm * BM + q * 32;
+            // the residual of the first 32 columns is on its way while the tile is computed
+            if (fetch && seg.nseg <= 1 && tn * BN + col_lo < p.Kout) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + col_lo);
+            if (!timed_wait_warp(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
                 if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_FULL); }
                 break;
             }
             tc_fence_after_sync();
-            const long long tile_row0 = (long long)tm * BM + q * 32;
             if (p.mode == 1) {
                 // Filter gradient: accumulator row = output channel k, columns = channels c of tap (r, s).
                 // The result lands in dw[k][r][s][c]; partial sums of different pixel ranges are added atomically.
@@ -628,8 +658,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                     __threadfence();
                     if (sizeof(T) == 4 && p.y_tma) {
 #pragma unroll 1
-                        for (int c32 = col_lo; c32 < col_hi && tn * BN + c32 < p.Kout; c32 += 32) {
+                        for (int c32 = col_lo; c32 < col_hi && tn * BN + c32 < p.Kout && res_ok; c32 += 32) {
                             float acc[32];
+                            if (fetch) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + c32);
 #pragma unroll
                             for (int j = 0; j < 32; j++) acc[j] = 0.f;
                             for (int c = seg.first_cta; c < seg.first_cta + seg.nseg; c++) {
@@ -640,7 +671,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                                     acc[4 * j] += v.x; acc[4 * j + 1] += v.y; acc[4 * j + 2] += v.z; acc[4 * j + 3] += v.w;
                                 }
                             }
-                            epilogue_store32(p, stage, acc, lane, tile_row0, tn * BN + c32);
+                            res_ok = epilogue_store32(p, stage, acc, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
+                            res_phase ^= 1u;
                         }
                     } else
 #pragma unroll 1
@@ -665,14 +697,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             }
 #pragma unroll 1
             for (int c32 = col_lo; c32 < col_hi; c32 += 32) {   // whole tile in one piece: straight to the output
-                if (tn * BN + c32 >= p.Kout) break;
+                if (tn * BN + c32 >= p.Kout || !res_ok) break;
+                if (fetch && c32 > col_lo) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + c32);
                 uint32_t r[32];
                 load_acc((uint32_t)(ab * BN + c32), r);
                 if (sizeof(T) == 4 && p.y_tma) {
                     float x[32];
 #pragma unroll
                     for (int j = 0; j < 32; j++) x[j] = __uint_as_float(r[j]);
-                    epilogue_store32(p, stage, x, lane, tile_row0, tn * BN + c32);
+                    res_ok = epilogue_store32(p, stage, x, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
+                    res_phase ^= 1u;
                     continue;
                 }
 #pragma unroll
@@ -687,7 +721,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl->tmem_empty[ab]);
         }
-        if (lane == 0) bulk_wait_group<0>();   // the slabs must outlive the copies that read them
+        if (!res_ok && !*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
+        if (lane == 0) bulk_wait_group_read<0>();   // the slabs must outlive the copies that read them
         if (p.debug && blockIdx.x == 0 && tid == 0) p.debug[0] = waited;
     } else if (warp == MMA_WARP) {
         // ------------------------------------------------------------ MMA issue (the warp as one, see elect_one)
@@ -1365,21 +1400,23 @@ static bool setup_tma(IgemmParams& p, int bn) {
 
 }  // namespace ob200
 
-// float32 outputs whose rows are whole 16-byte groups, stored in place and without a residual, leave by TMA stores.
+// float32 outputs whose rows are whole 16-byte groups and are stored in place leave by TMA stores.
 static void setup_tma_store(IgemmParams& p) {
     using namespace ob200;
     p.y_tma = 0;
     const TmaApi& api = tma_api();
-    if (!api.ok || p.mode != 0 || p.dtype == 1 || p.out_map || p.batch > 1 || p.residual || (p.Kout & 3)) return;
-    if (((uintptr_t)p.y | (uintptr_t)p.scale | (uintptr_t)p.shift) % 16) return;
+    if (!api.ok || p.mode != 0 || p.dtype == 1 || p.out_map || p.batch > 1 || (p.Kout & 3)) return;
+    if (((uintptr_t)p.y | (uintptr_t)p.residual | (uintptr_t)p.scale | (uintptr_t)p.shift) % 16) return;
     cuuint64_t dims[2] = {(cuuint64_t)p.Kout, (cuuint64_t)p.M};
     cuuint64_t strides[1] = {(cuuint64_t)p.Kout * 4};
     cuuint32_t box[2] = {32, 32};
     cuuint32_t steps[2] = {1, 1};
-    if (api.tiled(reinterpret_cast<CUtensorMap*>(p.tmap_y), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, p.y, dims, strides, box, steps,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-        p.y_tma = 1;
+    auto encode = [&](unsigned char* map, const void* base) {
+        return api.tiled(reinterpret_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box,
+                         steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (encode(p.tmap_y, p.y) && (!p.residual || encode(p.tmap_r, p.residual))) p.y_tma = 1;
 }
 
 static std::atomic<long long> g_tma_launches{0};

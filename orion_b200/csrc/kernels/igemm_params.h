@@ -91,6 +91,7 @@ typedef struct IgemmParams {
     unsigned long long mn_desc_bits;   /* filter gradient on TMA: the operand descriptors' bits above the address */
     int y_tma;         /* y is written by TMA stores (tmap_y: [M, Kout] in boxes of 32 x 32 float32) */
     OB200_ALIGN64 unsigned char tmap_y[128];
+    OB200_ALIGN64 unsigned char tmap_r[128];   /* the residual, in the same boxes */
     OB200_ALIGN64 unsigned char tmap_a[128];
     OB200_ALIGN64 unsigned char tmap_b[128];
 } IgemmParams;
