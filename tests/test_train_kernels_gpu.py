@@ -228,6 +228,38 @@ def test_multi_tensor_sgd_matches_torch(K):
             assert (a - b).abs().max().item() <= 2e-6 * max(1.0, b.abs().max().item()), step
 
 
+@pytest.mark.parametrize("N,H,C,Kout", [(2, 7, 4, 20), (3, 9, 24, 72), (5, 30, 12, 64), (1, 5, 28, 132), (2, 40, 16, 96), (1, 3, 32, 16)])
+def test_wgrad_1x1_with_few_channels(K, N, H, C, Kout):
+    """1x1 layers of fewer than 32 input channels: the input as a plain matrix whose copies reach past its rows, many splits of
+    few tiles, pixel counts that are no multiple of a k-block."""
+    torch.manual_seed(C + Kout)
+    x = torch.randn(N, H, H, C, device="cuda")
+    dy = torch.randn(N, H, H, Kout, device="cuda")
+    before = K.tma_launch_count()
+    dw = K.conv2d_wgrad_nhwc(x, dy, (1, 1), (1, 1), (0, 0))
+    assert K.tma_launch_count() > before and K.read_status() == 0
+    assert O.rel_err(dw, _wgrad_ref(x, dy, (1, 1), 1, 0, 1)) < TOL
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 4), (2, 2, 2, 8), (2, 3, 8, 12), (1, 16, 17, 20), (3, 9, 10, 36)])
+def test_depthwise_stride2_data_gradient_at_the_edges(K, shape):
+    """Odd and even heights and widths down to one pixel: the last dy row and column have no lower / right neighbour, the last dx
+    row and column may be missing."""
+    import torch.nn.functional as F
+    from orion_b200 import torch_ops
+    torch_ops.load()
+    Nb, H, W, C = shape
+    torch.manual_seed(H * 31 + W)
+    x = torch.randn(Nb, C, H, W, device="cuda").contiguous(memory_format=torch.channels_last).requires_grad_(True)
+    w = torch.randn(C, 1, 3, 3, device="cuda")
+    y = F.conv2d(x, w, None, 2, 1, 1, C)
+    dy = torch.randn_like(y)
+    y.backward(dy)
+    xd = x.detach().double().cpu().requires_grad_(True)
+    F.conv2d(xd, w.double().cpu(), None, 2, 1, 1, C).backward(dy.double().cpu())
+    assert O.rel_err(x.grad, xd.grad) < 1e-6   # at most four products per pixel
+
+
 @pytest.mark.parametrize("shape,stride", [((64, 56, 56, 144), 1), ((64, 112, 112, 96), 2), ((3, 9, 11, 8), 2), ((2, 7, 7, 960), 1),
                                           ((5, 10, 6, 32), 1)])
 def test_depthwise_backward_through_the_overrides(K, shape, stride):
