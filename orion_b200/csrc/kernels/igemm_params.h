@@ -64,6 +64,7 @@ typedef struct IgemmParams {
      * wg_cr columns each (wg_cr = C rounded up to 32), so dy is read once per wg_tpt taps.  wg_tpt <= 1: one tap
      * (and one channel block) per tile. */
     int wg_tpt, wg_cr;
+    int wg_plain;           /* 1x1 filter, stride 1, no padding: the layer input is copied as a plain [pixels, C] matrix */
     int bmul_h, bmul_w, badd_h, badd_w, step_h, step_w, div_h, div_w;
     /* Tap subset (TMA-fed launches only): the filter in memory has w_R x w_S taps and the launch iterates
      * R x S of them, tap (t, u) being filter tap (w_r0 + w_rstep*t, w_s0 + w_sstep*u).  w_R = 0: the launch
