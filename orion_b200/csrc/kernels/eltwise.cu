@@ -139,6 +139,8 @@ __global__ void __launch_bounds__(ELT_THREADS) maxpool_nhwc_f32_kernel(const flo
 // its channel quad, sharing the nine input columns they need (27 loads for four outputs instead of 36).
 __global__ void __launch_bounds__(ELT_THREADS) maxpool3x3s2_nhwc_f32_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                           int Nb, int H, int W, int C, int P, int Q, int pad) {
+    pdl_wait();
+    pdl_launch_dependents();
     pdl_launch_dependents();   // a convolution behind this kernel may set itself up meanwhile (pdl.cuh)
     const int c4 = C >> 2, qb_n = (Q + 3) / 4;
     const long long total = (long long)Nb * P * qb_n * c4;
@@ -236,6 +238,8 @@ __global__ void __launch_bounds__(ELT_THREADS) avgpool_nhwc_f32_kernel(const flo
 // HW rows over 8 thread rows (independent 16-byte loads, then a fixed-order sum through shared memory), so that even a
 // batch-4 request spreads over Nb * C / 128 CTAs instead of a handful.
 __global__ void __launch_bounds__(256) avgpool_nhwc_f32_v4_kernel(const float4* __restrict__ x, float4* __restrict__ y, int Nb, int HW, int C4) {
+    pdl_wait();
+    pdl_launch_dependents();
     __shared__ float4 sh[8][32];
     const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
     const int groups = (C4 + 31) / 32;
@@ -327,8 +331,8 @@ extern "C" int ob200_maxpool_nhwc_f32(const float* x, float* y, int Nb, int H, i
     if (k == 3 && stride == 2) {
         const long long total4 = (long long)Nb * P * ((Q + 3) / 4) * (C / 4);
         OB200_ELASTIC_HBM(maxpool3x3s2_nhwc_f32_kernel, ELT_CTAS_PER_SM);
-        maxpool3x3s2_nhwc_f32_kernel<<<elt_grid(total4, num_ctas), ELT_THREADS, 0, (cudaStream_t)stream>>>(x, y, Nb, H, W, C, P, Q, pad);
-        return (int)cudaGetLastError();
+        return launch_pdl(maxpool3x3s2_nhwc_f32_kernel, (unsigned)elt_grid(total4, num_ctas), ELT_THREADS, (cudaStream_t)stream, x, y, Nb, H, W, C, P, Q,
+                          pad);
     }
     long long total = (long long)Nb * P * Q * (C / 4);
     OB200_ELASTIC_HBM(maxpool_nhwc_f32_kernel, ELT_CTAS_PER_SM);
@@ -360,8 +364,8 @@ extern "C" int ob200_avgpool_nhwc_f32(const float* x, float* y, int Nb, int HW, 
     if ((C & 3) == 0 && ((uintptr_t)x | (uintptr_t)y) % 16 == 0) {
         const long long items = (long long)Nb * ((C / 4 + 31) / 32), cap = (long long)num_ctas * 8;
         OB200_ELASTIC_HBM(avgpool_nhwc_f32_v4_kernel, 8);
-        avgpool_nhwc_f32_v4_kernel<<<(int)(items < cap ? items : cap), 256, 0, (cudaStream_t)stream>>>((const float4*)x, (float4*)y, Nb, HW, C / 4);
-        return (int)cudaGetLastError();
+        return launch_pdl(avgpool_nhwc_f32_v4_kernel, (unsigned)(items < cap ? items : cap), 256, (cudaStream_t)stream, (const float4*)x, (float4*)y, Nb,
+                          HW, C / 4);
     }
     OB200_ELASTIC_HBM(avgpool_nhwc_f32_kernel, ELT_CTAS_PER_SM);
     avgpool_nhwc_f32_kernel<<<elt_grid((long long)Nb * C, num_ctas), ELT_THREADS, 0, (cudaStream_t)stream>>>(x, y, Nb, HW, C);
@@ -384,6 +388,8 @@ __global__ void pad_channels_kernel(const T* __restrict__ src, T* __restrict__ d
 }
 // float32, 3 -> 4 channels: one 16-byte store per pixel.
 __global__ void pad_channels_3to4_f32_kernel(const float* __restrict__ src, float4* __restrict__ dst, long long pixels) {
+    pdl_wait();
+    pdl_launch_dependents();
     for (long long px = (long long)blockIdx.x * blockDim.x + threadIdx.x; px < pixels; px += (long long)gridDim.x * blockDim.x) {
         const float* s = src + px * 3;
         dst[px] = make_float4(__ldg(s), __ldg(s + 1), __ldg(s + 2), 0.f);
@@ -398,7 +404,7 @@ extern "C" int ob200_pad_channels(const void* src, void* dst, long long pixels, 
     cudaStream_t s = (cudaStream_t)stream;
     OB200_HBM_BOUND();
     if (elem_bytes == 4 && C == 3 && Cpad == 4 && (uintptr_t)dst % 16 == 0)
-        ob200::pad_channels_3to4_f32_kernel<<<elt_grid(pixels, num_ctas), ELT_THREADS, 0, s>>>((const float*)src, (float4*)dst, pixels);
+        return ob200::launch_pdl(ob200::pad_channels_3to4_f32_kernel, (unsigned)ob200::elt_grid(pixels, num_ctas), ELT_THREADS, s, (const float*)src, (float4*)dst, pixels);
     else if (elem_bytes == 4)
         ob200::pad_channels_kernel<float><<<elt_grid(pixels * Cpad, num_ctas), ELT_THREADS, 0, s>>>((const float*)src, (float*)dst, pixels, C, Cpad);
     else
@@ -477,6 +483,8 @@ __global__ void __launch_bounds__(ELT_THREADS) depthwise3x3_nhwc_f32_kernel(
     const float* __restrict__ shift, int relu, int Nb, int H, int W, int C, int P, int Q, int pad_h, int pad_w, int w_tap_major,
     int flip) {
     // flip = 1 uses the filter rotated by 180 degrees: the data gradient of a stride-1 layer is this same convolution of dy
+    pdl_wait();
+    pdl_launch_dependents();
     constexpr int TW = 4, NCOL = (TW - 1) * STRIDE + 3;
     const int c4 = C / 4, qb_n = (Q + TW - 1) / TW;
     const long long total = (long long)Nb * P * qb_n * c4;
@@ -555,12 +563,11 @@ extern "C" int ob200_depthwise_conv2d_f32(const float* x, const float* w, float*
         OB200_ELASTIC_HBM(ob200::depthwise3x3_nhwc_f32_kernel<1>, 4);
         OB200_ELASTIC_HBM(ob200::depthwise3x3_nhwc_f32_kernel<2>, 4);
         if (stride_h == 1)
-            ob200::depthwise3x3_nhwc_f32_kernel<1><<<grid4, ELT_THREADS, 0, (cudaStream_t)stream>>>(x, w, y, scale, shift, relu, Nb, H, W, C, P,
-                                                                                                Q, pad_h, pad_w, w_tap_major, 0);
+            return ob200::launch_pdl(ob200::depthwise3x3_nhwc_f32_kernel<1>, grid4, ELT_THREADS, (cudaStream_t)stream, x, w, y, scale, shift, relu,
+                                     Nb, H, W, C, P, Q, pad_h, pad_w, w_tap_major, 0);
         else
-            ob200::depthwise3x3_nhwc_f32_kernel<2><<<grid4, ELT_THREADS, 0, (cudaStream_t)stream>>>(x, w, y, scale, shift, relu, Nb, H, W, C, P,
-                                                                                                Q, pad_h, pad_w, w_tap_major, 0);
-        return (int)cudaGetLastError();
+            return ob200::launch_pdl(ob200::depthwise3x3_nhwc_f32_kernel<2>, grid4, ELT_THREADS, (cudaStream_t)stream, x, w, y, scale, shift, relu,
+                                     Nb, H, W, C, P, Q, pad_h, pad_w, w_tap_major, 0);
     }
     const long long total = (long long)Nb * P * Q * (C / 4);
     // up to eight CTAs of 256 threads per granted SM: the kernel lives on loads in flight
@@ -619,13 +626,6 @@ __global__ void __launch_bounds__(ELT_THREADS) depthwise_dgrad_nhwc_f32_kernel(c
     }
 }
 
-// dw[c][r][s] = sum over output pixels of dy[n,p,q,c] * x[n, p*stride - pad + r, q*stride - pad + s, c]  (3x3 filters).
-// Threads are (channel quad, pixel lane); every thread keeps the 9 x 4 sums of its channel quad over the pixels it walks, a
-// shared-memory tree adds the lanes of a CTA and one atomicAdd per entry adds the CTAs (dw is cleared first).
-__global__ void __launch_bounds__(ELT_THREADS) depthwise_wgrad3x3_nhwc_f32_kernel(const float* __restrict__ dy, const float* __restrict__ x,
-                                                                                float* __restrict__ dw, int Nb, int H, int W, int C, int P,
-                                                                                int Q, int stride, int pad, int slabs) {
-    extern __shared__ float sh[];   // [blockDim.y][blockDim.x][36]
 // The stride-2 3x3 layers (padding 1): a thread owns two rows x eight columns of dx for four channels, which take two rows x five
 // columns of dy: ten 16-byte loads in flight and two coordinate divisions per sixteen outputs, filter in registers.  The general
 // kernel above pays four divisions, four scalar filter loads per tap and a dependent load chain per output.  HBM-bound:
@@ -696,6 +696,13 @@ __global__ void __launch_bounds__(ELT_THREADS, 2) depthwise_dgrad3x3s2_nhwc_f32_
     }
 }
 
+// dw[c][r][s] = sum over output pixels of dy[n,p,q,c] * x[n, p*stride - pad + r, q*stride - pad + s, c]  (3x3 filters).
+// Threads are (channel quad, pixel lane); every thread keeps the 9 x 4 sums of its channel quad over the pixels it walks, a
+// shared-memory tree adds the lanes of a CTA and one atomicAdd per entry adds the CTAs (dw is cleared first).
+__global__ void __launch_bounds__(ELT_THREADS) depthwise_wgrad3x3_nhwc_f32_kernel(const float* __restrict__ dy, const float* __restrict__ x,
+                                                                                float* __restrict__ dw, int Nb, int H, int W, int C, int P,
+                                                                                int Q, int stride, int pad, int slabs) {
+    extern __shared__ float sh[];   // [blockDim.y][blockDim.x][36]
     const int cq = blockDim.x, ry = blockDim.y;
     const int c_groups = (C / 4 + cq - 1) / cq;
     const int cg = blockIdx.x % c_groups, slab = blockIdx.x / c_groups;
