@@ -752,6 +752,25 @@ __global__ void __launch_bounds__(ELT_THREADS) depthwise_wgrad3x3_nhwc_f32_kerne
                             acc[r * 3 + sx][2] = fmaf(g[t].z, a.z, acc[r * 3 + sx][2]);
                             acc[r * 3 + sx][3] = fmaf(g[t].w, a.w, acc[r * 3 + sx][3]);
                         }
+                } else if (stride == 2) {
+                    // the nine distinct columns of the window at once; the general loop below waits for each of its twelve loads:
+                    // 112 x 112 x 96, batch 64: 263 -> 156 us
+                    float4 v[9];
+#pragma unroll
+                    for (int j = 0; j < 9; j++)
+                        v[j] = (unsigned)(w0 + j) < (unsigned)W ? __ldg(reinterpret_cast<const float4*>(xrow + (long long)(w0 + j) * C))
+                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int t = 0; t < 4; t++)
+#pragma unroll
+                        for (int sx = 0; sx < 3; sx++) {
+                            if ((unsigned)(w0 + 2 * t + sx) >= (unsigned)W) continue;
+                            const float4 a = v[2 * t + sx];
+                            acc[r * 3 + sx][0] = fmaf(g[t].x, a.x, acc[r * 3 + sx][0]);
+                            acc[r * 3 + sx][1] = fmaf(g[t].y, a.y, acc[r * 3 + sx][1]);
+                            acc[r * 3 + sx][2] = fmaf(g[t].z, a.z, acc[r * 3 + sx][2]);
+                            acc[r * 3 + sx][3] = fmaf(g[t].w, a.w, acc[r * 3 + sx][3]);
+                        }
                 } else {
 #pragma unroll
                     for (int t = 0; t < 4; t++)
