@@ -736,8 +736,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         // ------------------------------------------------------------ MMA issue (the warp as one, see elect_one)
         // A TMA-fed filter gradient keeps both operands the way they lie in memory (pixel-major, i.e.
         // MN-major for this GEMM); everything else stages K-major rows.
-        const bool mn_major = !ATMEM && p.mode == 1 && p.use_tma;
-        const uint32_t idesc = umma_idesc(sizeof(T) == 4 ? 2 : 1, BM, BN) | (mn_major ? (UMMA_IDESC_A_MN | UMMA_IDESC_B_MN) : 0u);
+        // (With the activation parts in tensor memory only the other operand is.)
+        const bool mn_major = p.mode == 1 && p.use_tma;
+        const uint32_t idesc = umma_idesc(sizeof(T) == 4 ? 2 : 1, BM, BN) | (mn_major ? ((ATMEM ? 0u : UMMA_IDESC_A_MN) | UMMA_IDESC_B_MN) : 0u);
         const uint64_t kstep = mn_major ? (1024 >> 4) : (32 >> 4);   // descriptor address advance per k-step of 8 (16 for bf16)
         // operand descriptor above the address
         const uint64_t desc_bits = mn_major ? p.mn_desc_bits : umma_desc_sw128(0);
@@ -782,7 +783,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                             const uint32_t ta_hi = tmem_base + C::A_TMEM_COL0 + s * 64, ta_lo = ta_hi + 32;
 #pragma unroll
                             for (int ks = 0; ks < 4; ks++) {
-                                const uint64_t o = (uint64_t)ks * (32 >> 4);
+                                const uint64_t o = (uint64_t)ks * kstep;
                                 umma_tf32_ts(dx, ta_lo + ks * 8, b_hi + o, idesc, ks > 0 ? 1u : first);
                                 umma_tf32_ts(dx, ta_hi + ks * 8, b_lo + o, idesc, 1u);
                                 umma_tf32_ts(d, ta_hi + ks * 8, b_hi + o, idesc, ks > 0 ? 1u : first_hh);
@@ -860,8 +861,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                             uint32_t hi[16], lo[16];
 #pragma unroll
                             for (int j = 0; j < 4; j++) {
-                                const float4 v = *reinterpret_cast<const float4*>(a_hi + sw128_offset(row, (uint32_t)(c0 / 4 + j)));
-                                const float e[4] = {v.x, v.y, v.z, v.w};
+                                float e[4];
+                                if (p.mode == 1) {
+                                    // dy tile of a filter gradient: boxes of 32 pixels x 32 channels (128-byte swizzle of 32-byte
+                                    // atoms), this thread's row is a channel: one value per pixel, 128 bytes per warp read
+#pragma unroll
+                                    for (int k = 0; k < 4; k++) {
+                                        const uint32_t px = (uint32_t)(c0 + 4 * j + k);
+                                        e[k] = *reinterpret_cast<const float*>(a_hi + q * 4096 + px * 128 + ((((uint32_t)lane >> 3) ^ (px & 3u)) << 5) +
+                                                                               (lane & 7) * 4);
+                                    }
+                                } else {
+                                    const float4 v = *reinterpret_cast<const float4*>(a_hi + sw128_offset(row, (uint32_t)(c0 / 4 + j)));
+                                    e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
+                                }
 #pragma unroll
                                 for (int k = 0; k < 4; k++) {
                                     // Round to nearest on this side (it costs nothing here): the remainder is then
@@ -1454,7 +1467,7 @@ extern "C" int ob200_igemm_launch(const IgemmParams* params, int bn, int num_cta
         const char* e = getenv("ORION_A_TMEM");
         return e && e[0] == '0';
     }();
-    p.a_in_tmem = (p.dtype == 0 && p.mode == 0 && !a_tmem_off) ? 1 : 0;
+    p.a_in_tmem = (p.dtype == 0 && p.mode == 0 && !a_tmem_off) ? 1 : 0;   // filter gradients: below, where TMA feeds them
     {   // Cross-term accumulator where no CTA of a whole-device launch computes more than two pieces (see
         // IgemmParams::cross_acc); decided from the problem and the device, not from this call's CTA count, so that the
         // arithmetic does not change with the SM quota.  ORION_CROSS_ACC=0/1 pins it.
@@ -1470,8 +1483,14 @@ extern "C" int ob200_igemm_launch(const IgemmParams* params, int bn, int num_cta
         const long long units = (long long)p.tiles_m * p.tiles_n * (p.splits > 1 ? p.splits : 1) * (p.batch > 1 ? p.batch : 1);
         p.cross_acc = (p.a_in_tmem && (force == '1' || (force != '0' && !p.stream_k && units <= 2LL * device_sms))) ? 1 : 0;
     }
-    if (setup_tma(p, bn)) g_tma_launches.fetch_add(1, std::memory_order_relaxed);
-    else if (p.require_tma || p.w_R > 0) return -4;   // tap subsets exist only on the TMA path
+    if (setup_tma(p, bn)) {
+        g_tma_launches.fetch_add(1, std::memory_order_relaxed);
+        // A filter gradient's dy parts in tensor memory take a third off its shared-memory traffic per k-block (192 -> 128 KB of
+        // a 128 x 128 x 32 one), which is what bounds it: 3x3 64 -> 64 at
+        // 56 x 56, batch 32 145 -> 121 us, 3x3 256 -> 256 at 14 x 14 72 -> 61 us.
+        if (p.dtype == 0 && p.mode == 1 && !a_tmem_off) p.a_in_tmem = 1;
+    }
+    if (!p.use_tma && (p.require_tma || p.w_R > 0)) return -4;   // tap subsets exist only on the TMA path
     setup_tma_store(p);
     {   // class of this launch for the scheduler's profiles: arithmetic intensity of the problem against the device's
         const double batch = p.batch > 1 ? p.batch : 1;
