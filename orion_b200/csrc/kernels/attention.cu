@@ -10,6 +10,8 @@
 // maximum.  Bound: the exponentials (16 per clock and SM; the two products of a step take a third of that time), so what
 // counts is that twelve softmax warps per SM always have scores to work on: scores and output of one item take 128
 // tensor-memory columns and 66 KB of shared memory, and three items share an SM.
+// 8 x 384 x 12 heads: 33.1 us with all scores of a query tile in tensor memory (one item per SM, two passes over them), 15.0 now;
+// 16 x 512 x 16 heads, causal, in three launches: 43 us.
 // Every wait is bounded; on expiry the kernel sets the status word, frees tensor memory and returns.
 #include <cuda.h>
 #include <cuda_bf16.h>

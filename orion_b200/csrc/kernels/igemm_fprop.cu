@@ -856,37 +856,41 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                         const int q = warp & 3;
                         const uint32_t row = (uint32_t)(q * 32 + lane);
                         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + C::A_TMEM_COL0 + s * 64;
+auto split_row = [&](auto load4) {   // load4(i): values 4i .. 4i+3 of this thread's row
 #pragma unroll
-                        for (int c0 = 0; c0 < 32; c0 += 16) {
-                            uint32_t hi[16], lo[16];
+                            for (int c0 = 0; c0 < 32; c0 += 16) {
+                                uint32_t hi[16], lo[16];
 #pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                float e[4];
-                                if (p.mode == 1) {
-                                    // dy tile of a filter gradient: boxes of 32 pixels x 32 channels (128-byte swizzle of 32-byte
-                                    // atoms), this thread's row is a channel: one value per pixel, 128 bytes per warp read
+                                for (int j = 0; j < 4; j++) {
+                                    const float4 v = load4(c0 / 4 + j);
+                                    const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
                                     for (int k = 0; k < 4; k++) {
-                                        const uint32_t px = (uint32_t)(c0 + 4 * j + k);
-                                        e[k] = *reinterpret_cast<const float*>(a_hi + q * 4096 + px * 128 + ((((uint32_t)lane >> 3) ^ (px & 3u)) << 5) +
-                                                                               (lane & 7) * 4);
+                                        // Round to nearest on this side (it costs nothing here): the remainder is then
+                                        // zero-mean, so the dropped lo*lo product carries no bias even though the filter
+                                        // side splits by truncation.
+                                        const uint32_t h = __float_as_uint(tf32_round_bits(e[k])) & 0xffffe000u;
+                                        hi[4 * j + k] = h;
+                                        lo[4 * j + k] = __float_as_uint(tf32_round_bits(e[k] - __uint_as_float(h)));
                                     }
-                                } else {
-                                    const float4 v = *reinterpret_cast<const float4*>(a_hi + sw128_offset(row, (uint32_t)(c0 / 4 + j)));
-                                    e[0] = v.x; e[1] = v.y; e[2] = v.z; e[3] = v.w;
                                 }
-#pragma unroll
-                                for (int k = 0; k < 4; k++) {
-                                    // Round to nearest on this side (it costs nothing here): the remainder is then
-                                    // zero-mean, so the dropped lo*lo product carries no bias even though the filter
-                                    // side splits by truncation.
-                                    const uint32_t h = __float_as_uint(tf32_round_bits(e[k])) & 0xffffe000u;
-                                    hi[4 * j + k] = h;
-                                    lo[4 * j + k] = __float_as_uint(tf32_round_bits(e[k] - __uint_as_float(h)));
-                                }
+                                tmem_st_32x16(t_row + c0, hi);
+                                tmem_st_32x16(t_row + 32 + c0, lo);
                             }
-                            tmem_st_32x16(t_row + c0, hi);
-                            tmem_st_32x16(t_row + 32 + c0, lo);
+                        };
+                        if (p.mode == 1) {
+                            // dy tile of a filter gradient: boxes of 32 pixels x 32 channels (128-byte swizzle of 32-byte atoms),
+                            // this thread's row is a channel: one value per pixel, 128 bytes per warp read
+                            const uint8_t* box = a_hi + q * 4096 + (lane & 7) * 4;
+                            split_row([&](int i) {
+                                float e[4];
+#pragma unroll
+                                for (int k = 0; k < 4; k++)   // pixel 4i + k: its atoms are XORed with k
+                                    e[k] = *reinterpret_cast<const float*>(box + (4 * i + k) * 128 + ((((uint32_t)lane >> 3) ^ (uint32_t)k) << 5));
+                                return make_float4(e[0], e[1], e[2], e[3]);
+                            });
+                        } else {
+                            split_row([&](int i) { return *reinterpret_cast<const float4*>(a_hi + sw128_offset(row, (uint32_t)i)); });
                         }
                         tmem_st_wait();
                         tc_fence_before_sync();
@@ -1487,7 +1491,7 @@ extern "C" int ob200_igemm_launch(const IgemmParams* params, int bn, int num_cta
         g_tma_launches.fetch_add(1, std::memory_order_relaxed);
         // A filter gradient's dy parts in tensor memory take a third off its shared-memory traffic per k-block (192 -> 128 KB of
         // a 128 x 128 x 32 one), which is what bounds it: 3x3 64 -> 64 at
-        // 56 x 56, batch 32 145 -> 121 us, 3x3 256 -> 256 at 14 x 14 72 -> 61 us.
+        // 56 x 56, batch 32 155 -> 121 us, 3x3 256 -> 256 at 14 x 14 75 -> 61 us (integer rounding in the splitters included).
         if (p.dtype == 0 && p.mode == 1 && !a_tmem_off) p.a_in_tmem = 1;
     }
     if (!p.use_tma && (p.require_tma || p.w_R > 0)) return -4;   // tap subsets exist only on the TMA path
