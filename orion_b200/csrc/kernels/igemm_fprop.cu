@@ -58,7 +58,7 @@ constexpr int PROD_WARPS = 8;     // warps 9-16 when the operands are gathered w
 constexpr int TMA_WARP = 17;      // one lane issues the TMA copies of TMA-fed launches
 constexpr int NTHREADS = 18 * 32;
 
-// ATMEM: 3xTF32 with both parts of the activation tile in tensor memory (forward / data gradient / GEMM).
+// ATMEM: 3xTF32 with both parts of the activation tile in tensor memory (the activation of forward, data gradient and GEMM, dy of a TMA-fed filter gradient).
 template <typename T, int BN, int PASSES, bool ATMEM>
 struct Cfg {
     static constexpr bool kSplit = sizeof(T) == 4 && PASSES == 3;   // 3xTF32; PASSES == 1 is plain TF32

@@ -80,7 +80,7 @@ typedef struct IgemmParams {
      * ow*bmul_w + tma_base_w) and whose per-tap offsets are non-negative, the filter through a tiled map
      * over [batch, Kout, R, S, C].  0: the producer warps gather with 16-byte asynchronous copies. */
     int use_tma;
-    int a_in_tmem;     /* 3xTF32, mode 0: the splitters put both parts of the activation tile into tensor memory */
+    int a_in_tmem;     /* 3xTF32, mode 0 or TMA-fed mode 1: the splitters put both parts of the first operand tile into tensor memory */
     /* 3xTF32 with a_in_tmem: the two small cross products (lo*hi, hi*lo) accumulate in a second accumulator and are
      * added to the main one in the epilogue.  The tensor core adds into its fp32 accumulator by truncation; with the
      * cross terms elsewhere the large accumulator takes one addition per k-step instead of three, which cuts the
