@@ -350,7 +350,10 @@ __device__ __forceinline__ bool epilogue_store32(const IgemmParams& p, float* sl
         }
     }
     if (p.residual) {
-        if (!mbar_wait_warp(res_bar, res_phase, abort_flag)) return false;
+        if (!mbar_wait_warp(res_bar, res_phase, abort_flag)) {
+            if (!*abort_flag) { *abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
+            return false;
+        }
 #pragma unroll
         for (int ch = 0; ch < 8; ch++) {
             const float4 v = *reinterpret_cast<const float4*>(row + ((ch ^ (lane & 7)) << 4));
@@ -546,7 +549,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         const int q = warp & 3;
         const int grp = epi_id >> 2;
         const int col_lo = grp * (BN / epi_groups), col_hi = col_lo + BN / epi_groups;
-        const int epi_threads = 128 * epi_groups;
         float* stage = epi_stage + epi_id * 1024;
         const int sub = lane >> 2;          // row within a group of eight
         const int cc = (lane & 3) * 4;      // first of this lane's four channels within a 16-channel chunk
@@ -571,11 +573,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         const bool fetch = sizeof(T) == 4 && p.y_tma && p.residual != nullptr;
         uint64_t* res_bar = &ctl->res_full[epi_id];
         uint32_t res_phase = 0;
-        bool res_ok = true;
+        // The epilogue warps meet three times per piece of a cut tile, at a named barrier, which has no limit of its own.  So a
+        // warp that has given up (`ok` is false) stays in the loop and meets the others for every such piece until the work is
+        // walked; they get there too, since their own waits run out or see the abort flag.  (Bounded waits on a shared-memory
+        // barrier instead: 0.7 us more for each layer of cut tiles.)
+        const int epi_threads = 128 * epi_groups;
+        auto meet = [&] { asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory"); };
+        bool ok = true;
         int local = 0;
         WorkIter work(p, tiles);
         Seg seg;
-        for (; res_ok && work.next(seg); local++) {
+        for (; work.next(seg); local++) {
             const int tile = seg.tile;
             const int bidx = tile / tiles_per_problem;
             const int tloc = tile - bidx * tiles_per_problem;
@@ -586,10 +594,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             const uint32_t acc_use = cross ? (uint32_t)local : (uint32_t)(local >> 1);
             const long long tile_row0 = (long long)tm * BM + q * 32;
             // the residual of the first 32 columns is on its way while the tile is computed
-            if (fetch && seg.nseg <= 1 && tn * BN + col_lo < p.Kout) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + col_lo);
-            if (!timed_wait_warp(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
+            if (fetch && ok && seg.nseg <= 1 && tn * BN + col_lo < p.Kout) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + col_lo);
+            if (!ok || !timed_wait_warp(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
+                ok = false;
                 if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_FULL); }
-                break;
+                if (seg.nseg > 1 && p.mode == 0) { meet(); meet(); meet(); }
+                continue;
             }
             tc_fence_after_sync();
             if (p.mode == 1) {
@@ -655,18 +665,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ctl->tmem_empty[ab]);   // the accumulator is out of TMEM
                 __threadfence();
-                asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory");
+                meet();
                 if (tid == 0) {
                     int prev = atomicAdd(p.counters + seg.slot, 1);
                     ctl->last_flag = (prev == seg.nseg - 1);
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory");
+                meet();
                 if (ctl->last_flag) {
                     // Last piece to arrive: every slab of the tile is published.  Sum them in CTA (split) order.
                     __threadfence();
                     if (sizeof(T) == 4 && p.y_tma) {
 #pragma unroll 1
-                        for (int c32 = col_lo; c32 < col_hi && tn * BN + c32 < p.Kout && res_ok; c32 += 32) {
+                        for (int c32 = col_lo; c32 < col_hi && tn * BN + c32 < p.Kout && ok; c32 += 32) {
                             float acc[32];
                             if (fetch) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + c32);
 #pragma unroll
@@ -679,8 +689,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                                     acc[4 * j] += v.x; acc[4 * j + 1] += v.y; acc[4 * j + 2] += v.z; acc[4 * j + 3] += v.w;
                                 }
                             }
-                            res_ok = epilogue_store32(p, stage, acc, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
-                            res_phase ^= 1u;
+                            ok = epilogue_store32(p, stage, acc, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
+                            res_phase ^= (uint32_t)ok;
                         }
                     } else
 #pragma unroll 1
@@ -700,12 +710,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                     }
                     if (tid == 0) p.counters[seg.slot] = 0;
                 }
-                asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory");   // last_flag is rewritten by the next piece
+                meet();   // last_flag is rewritten by the next piece
                 continue;
             }
 #pragma unroll 1
             for (int c32 = col_lo; c32 < col_hi; c32 += 32) {   // whole tile in one piece: straight to the output
-                if (tn * BN + c32 >= p.Kout || !res_ok) break;
+                if (tn * BN + c32 >= p.Kout || !ok) break;
                 if (fetch && c32 > col_lo) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + c32);
                 uint32_t r[32];
                 load_acc((uint32_t)(ab * BN + c32), r);
@@ -713,8 +723,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                     float x[32];
 #pragma unroll
                     for (int j = 0; j < 32; j++) x[j] = __uint_as_float(r[j]);
-                    res_ok = epilogue_store32(p, stage, x, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
-                    res_phase ^= 1u;
+                    ok = epilogue_store32(p, stage, x, res_bar, res_phase, abort_flag, lane, tile_row0, tn * BN + c32);
+                    res_phase ^= (uint32_t)ok;
                     continue;
                 }
 #pragma unroll
@@ -729,7 +739,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl->tmem_empty[ab]);
         }
-        if (!res_ok && !*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
+        if (!ok && fetch) mbar_wait_landed(res_bar, res_phase);   // a residual copy may still be under way: the slab must outlive it
         if (lane == 0) bulk_wait_group_read<0>();   // the slabs must outlive the copies that read them
         if (p.debug && blockIdx.x == 0 && tid == 0) p.debug[0] = waited;
     } else if (warp == MMA_WARP) {

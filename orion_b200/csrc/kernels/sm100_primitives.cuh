@@ -81,6 +81,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
+// For a role that gives up with copies of its own under way: they must land before the CTA leaves its shared memory.  Bounded, but
+// blind to the abort flag, which is up already.
+__device__ __forceinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try_wait_hint(bar, parity, 4000u))
+        if (clock64() - t0 > OB200_WAIT_CYCLES) return;
+}
+
 // The same for a whole converged warp: every lane gets the same answer, so that a wait which runs out unwinds the warp as one.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
