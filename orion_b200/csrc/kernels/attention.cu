@@ -41,8 +41,8 @@ struct AttnParams {
     int* status;
     int B, S, H;
     int causal;
-    int negate;            // scale < 0: the scores change sign before the softmax
-    float scale_log2;      // |scale| * log2(e)
+    float factor;          // what the scores are multiplied by ahead of the mask: 1, or -1 / 0 for a negative / zero scale
+    float scale_log2;      // |scale| * log2(e); 1 for a zero scale, so that a masked score stays -infinity
     int q_tiles;           // ceil(S / 128)
     int first, last;       // work items [first, last) of this launch
     alignas(64) unsigned char tmap[128];   // qkv as [B][S][3H][64], boxes of 64 rows
@@ -232,9 +232,9 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ctl->s_free);
-                if (p.negate) {
+                if (p.factor != 1.f) {
 #pragma unroll
-                    for (int j = 0; j < AT_KEYS; j++) x[j] = -x[j];
+                    for (int j = 0; j < AT_KEYS; j++) x[j] *= p.factor;
                 }
                 const int left = key_end - t * AT_KEYS;
                 if (left < AT_KEYS) {
@@ -370,8 +370,8 @@ extern "C" int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* l
     p.status = ob200_status_word_for_current_device();
     p.B = B; p.S = S; p.H = H;
     p.causal = causal ? 1 : 0;
-    p.negate = scale < 0.f ? 1 : 0;
-    p.scale_log2 = (scale < 0.f ? -scale : scale) * 1.4426950408889634f;
+    p.factor = scale < 0.f ? -1.f : scale == 0.f ? 0.f : 1.f;
+    p.scale_log2 = scale == 0.f ? 1.f : (scale < 0.f ? -scale : scale) * 1.4426950408889634f;
     p.q_tiles = (S + AT_QROWS - 1) / AT_QROWS;
     const long long all = (long long)B * H * p.q_tiles;
     if (all > 0x3fffffffLL) return -1;

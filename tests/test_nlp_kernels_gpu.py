@@ -191,6 +191,23 @@ def test_long_attention_matches_float64(tops, B, S, H, causal, spread, scale):
     assert O.rel_err(ctx, want) < 1e-2
 
 
+@pytest.mark.parametrize("B,S,H,causal", [(2, 384, 3, True), (1, 77, 2, False), (2, 100, 2, True), (1, 128, 1, False), (1, 1, 1, True)])
+def test_attention_with_a_zero_scale_is_the_mean_of_the_keys_that_count(tops, B, S, H, causal):
+    """All scores equal: every key up to the query (causal) or the sequence's end weighs the same, masked ones nothing."""
+    from orion_b200 import kernels
+    torch.manual_seed(7 + S)
+    qkv = torch.randn(B, S, 3 * H * 64, device="cuda").to(torch.bfloat16)
+    v = qkv.double().cpu().view(B, S, 3, H, 64)[:, :, 2]
+    want = v.cumsum(1) / torch.arange(1, S + 1).view(1, S, 1, 1) if causal else v.mean(1, keepdim=True).expand_as(v)
+    got = [tops.attention(qkv, H, 0.0, causal)]
+    if S % 8 == 0:
+        got.append(tops.attention_long(qkv, H, 0.0, causal))
+    assert kernels.read_status() == 0
+    for ctx in got:
+        # the weights are exact, the sums float32; the output is rounded to bfloat16 (2^-9)
+        assert O.rel_err(ctx.view(B, S, H, 64), want) < 4e-3
+
+
 # ---------------------------------------------------------------------------------------------- training on the own GEMM
 @pytest.mark.parametrize("rows,K,N,bias,res", [(3072, 768, 2304, True, False), (3072, 768, 768, True, True), (520, 256, 136, False, True),
                                                (64, 3072, 768, True, True), (8192, 1024, 1024, False, False)])
