@@ -16,6 +16,7 @@
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <float.h>
 #include <stdint.h>
 #include <stdlib.h>
 #include <string.h>
@@ -250,7 +251,7 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
                 // 2^AT_RESCALE: float32 has the range, and the output in tensor memory is hardly ever read back.
                 bool waited = false;
                 if (t == 0) {
-                    m_ref = top;
+                    m_ref = fmaxf(top, -FLT_MAX);   // finite where all scores so far are -infinity: they weigh nothing, unless no other follows
                 } else if (__any_sync(0xffffffffu, top > m_ref + AT_RESCALE)) {
                     const bool grow = top > m_ref + AT_RESCALE;
                     const float f = grow ? exp2_approx(m_ref - top) : 1.f;

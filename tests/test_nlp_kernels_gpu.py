@@ -208,6 +208,28 @@ def test_attention_with_a_zero_scale_is_the_mean_of_the_keys_that_count(tops, B,
         assert O.rel_err(ctx.view(B, S, H, 64), want) < 4e-3
 
 
+@pytest.mark.parametrize("S,dead,causal", [(200, 64, False), (200, 130, True), (384, 70, False), (128, 128, False), (64, 3, False)])
+def test_attention_over_leading_keys_with_infinite_scores(tops, S, dead, causal):
+    """Scores of -infinity weigh nothing, also where they fill the first 64-key steps of a row; a row that has no other score has
+    no softmax (NaN)."""
+    from orion_b200 import kernels
+    torch.manual_seed(S + dead)
+    qkv = torch.randn(1, S, 3, 2, 64, device="cuda").to(torch.bfloat16)
+    qkv[:, :, 0] = qkv[:, :, 0].abs() + 0.125
+    qkv[:, :dead, 1] = -float("inf")
+    ctx = tops.attention(qkv.view(1, S, -1), 2, 0.125, causal).view(1, S, 2, 64).double().cpu()
+    assert kernels.read_status() == 0
+    q, k, v = qkv.double().cpu().permute(2, 0, 3, 1, 4)
+    scores = q @ k.transpose(-1, -2) * 0.125
+    if causal:
+        scores = scores.masked_fill(torch.ones(S, S, dtype=torch.bool).triu(1), -float("inf"))
+    want = (scores.softmax(-1) @ v).permute(0, 2, 1, 3)
+    assert torch.equal(ctx.isnan(), want.isnan())
+    if not want.isnan().all():
+        # as in the tests above: bfloat16 probabilities and output
+        assert O.rel_err(ctx[~want.isnan()], want[~want.isnan()]) < 2e-2
+
+
 # ---------------------------------------------------------------------------------------------- training on the own GEMM
 @pytest.mark.parametrize("rows,K,N,bias,res", [(3072, 768, 2304, True, False), (3072, 768, 768, True, True), (520, 256, 136, False, True),
                                                (64, 3072, 768, True, True), (8192, 1024, 1024, False, False)])
