@@ -149,6 +149,10 @@ int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const float* bias,
                        int N, int K, int a_mn, int b_mn, long long lda, long long ldb, long long ldc, int batch_inner,
                        int batch_outer, long long a_si, long long a_so, long long b_si, long long b_so, long long c_si,
                        long long c_so, float alpha, int out_f32, int tri, int num_ctas, void* stream);
+/* How such a call is cut up (host logic only): tile width, CTAs that share a tile of 128 rows each (1, or a pair), split-K factor
+ * (before the limit of the stream's scratch) and grid.  The split factor is the same for every num_ctas. */
+int ob200_plan_gemm_bf16(int M, int N, int K, long long batch, int tri, int num_ctas, int* bn_out, int* ctas_per_tile_out,
+                         int* splits_out, int* grid_out);
 
 /* out[col] = sum over rows of x[row, col] (rows `ld` elements apart), summed in a fixed order: the bias gradient of a linear
  * layer.  dtype 0 float32, 1 bfloat16.  Stands where the reference's clients launch ATen's reduce_kernel

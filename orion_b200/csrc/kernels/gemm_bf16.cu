@@ -494,6 +494,57 @@ static bool gm_make_map(unsigned char* out, const void* base, long long inner, l
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Tile width, CTAs per tile and split factor of a problem.
+//
+// The smallest modelled time in microseconds: rounds of tiles, each as long as its k-blocks or as a tile's way out of tensor
+// memory, whichever is longer, the way out of the last one, and for pairs the start of a launch in clusters.  Split-K (few tiles,
+// long reduction) adds the second launch and writing and reading the partial matrices at about 6 TB/s.  The constants are a fit
+// to 359 shapes (16 - 8192 tokens times the widths of the clients' layers in all three layouts, and batched attention products),
+// each measured in every tiling: the choice is 0.3 % slower than the fastest tiling of the same split on average, 7 % at worst.
+// A model of k-blocks alone took pairs where the way out bounds (64-deep products 512 x 512 x 256 problems: 54.2 us, 43.3 in single
+// CTAs; 3072 x 1024 over 72 tokens 6.9, 6.2) and cut reductions that one round of 128-wide tiles had held (2048 x 768 x 3072: 34.5 us,
+// 16.0 now; 3072 x 768 x 8192: 56.3, 33.7): where 128 x 128 tiles fill more than half of the device nothing is cut.
+//
+// The split is planned for the device's SM count, never for the quota of the call, so the summation order (and the result, bit for
+// bit) is the same for every quota.
+struct GemmPlan { int bn, cg, splits, grid; };
+struct GemmTile { int bn, cg; double kblock_us, tile_us, tail_us, launch_us; };
+static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int device_sms, int num_ctas) {
+    static const GemmTile kNarrow = {64, 1, 0.44, 2.15, 1.0, 0.0};   // outputs of at most 64 columns
+    static const GemmTile kTiles[] = {{128, 1, 0.44, 2.15, 1.0, 0.0}, {256, 1, 0.51, 3.0, 2.0, 0.0},
+                                      {128, 2, 0.32, 2.15, 1.0, 1.8}, {256, 2, 0.45, 3.0, 2.0, 1.8}};
+    const GemmTile* list = N <= 64 ? &kNarrow : kTiles;
+    const int count = N <= 64 ? 1 : 4;
+    const long long kblocks = (K + GM_BK - 1) / GM_BK;
+    auto tiles_of = [&](int bn, int cg) { return batch * (((long long)M + cg * GM_BM - 1) / (cg * GM_BM)) * (((long long)N + bn - 1) / bn); };
+    auto fits = [&](const GemmTile& t) { return !((t.bn == 256 && N < 256) || (t.cg == 2 && (M <= GM_BM || tri != 0))); };
+    auto price = [&](const GemmTile& t, int splits, long long at_once) {
+        const double rounds = (double)((tiles_of(t.bn, t.cg) * splits + at_once - 1) / at_once);
+        const double depth = (double)((kblocks + splits - 1) / splits) * t.kblock_us;
+        const double us = t.launch_us + rounds * (depth > t.tile_us ? depth : t.tile_us) + t.tail_us;
+        return splits > 1 ? us + 6.0 + (double)splits * batch * M * N * 8.0 / 6e6 : us;
+    };
+    const bool may_split = tiles_of(list[0].bn, 1) * 2 <= device_sms && kblocks >= 8 && tri == 0;
+    GemmPlan pl = {0, 1, 1, 1};
+    double best = 0.0;
+    for (int i = 0; i < count; i++) {
+        const GemmTile& t = list[i];
+        const long long at_once = device_sms / t.cg, tiles = tiles_of(t.bn, t.cg);
+        if (!fits(t) || at_once < 1) continue;
+        long long sp = 1;
+        if (may_split && tiles * 2 <= at_once) {
+            sp = at_once / tiles;
+            if (sp > kblocks / 4) sp = kblocks / 4;
+            if (sp > 16) sp = 16;
+        }
+        const double us = price(t, (int)sp, at_once);
+        if (pl.bn == 0 || us < best) { best = us; pl.bn = t.bn; pl.cg = t.cg; pl.splits = (int)sp; }
+    }
+    const long long ctas = tiles_of(pl.bn, pl.cg) * pl.splits * pl.cg, most = pl.cg == 2 ? (num_ctas < 2 ? 2 : num_ctas & ~1) : num_ctas;   // whole pairs
+    pl.grid = (int)(ctas < most ? ctas : most);
+    return pl;
+}
+
 template <int BN, int CG>
 static int gm_launch(const GemmParams& p, int grid, cudaStream_t stream) {
     static bool attr_set[64] = {};
@@ -511,7 +562,6 @@ static int gm_launch(const GemmParams& p, int grid, cudaStream_t stream) {
         const char* e = getenv("ORION_PDL");
         return !(e && e[0] == '0');
     }();
-    if (CG == 2) grid = grid < 2 ? 2 : grid & ~1;   // whole pairs
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = dim3((unsigned)grid);
@@ -541,6 +591,18 @@ static int gm_launch(const GemmParams& p, int grid, cudaStream_t stream) {
 extern "C" int* ob200_status_word_for_current_device(void);
 extern "C" float* ob200_stream_slabs(void* stream, size_t* bytes);
 extern "C" int ob200_plan_sm_count(void);
+
+// See include/orion_kernels.h.
+extern "C" int ob200_plan_gemm_bf16(int M, int N, int K, long long batch, int tri, int num_ctas, int* bn_out, int* ctas_per_tile_out,
+                                    int* splits_out, int* grid_out) {
+    if (M <= 0 || N <= 0 || K <= 0 || batch <= 0 || tri < 0 || tri > 3 || num_ctas <= 0) return -1;
+    const ob200::GemmPlan pl = ob200::gm_plan(M, N, K, batch, tri, ob200_plan_sm_count(), num_ctas);
+    if (bn_out) *bn_out = pl.bn;
+    if (ctas_per_tile_out) *ctas_per_tile_out = pl.cg;
+    if (splits_out) *splits_out = pl.splits;
+    if (grid_out) *grid_out = pl.grid;
+    return 0;
+}
 
 // See include/orion_kernels.h.  Returns 0, -1 (unsupported sizes), -2 (misaligned pointers or strides), -4 (no TMA descriptor).
 extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const float* bias, const void* bias_bf16, const void* residual,
@@ -585,32 +647,9 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
     p.vec_ok = ((uintptr_t)c % 16 == 0) && ((uintptr_t)residual % 16 == 0) && (!residual || !out_f32) && (ldc % cal == 0) && (batch_inner == 1 || c_si % cal == 0) && (batch_outer == 1 || c_so % cal == 0);
     const int plan = ob200_plan_sm_count();
     p.kblocks = (K + GM_BK - 1) / GM_BK;
-    // Tile and split: the smallest modelled time, in hundredths of what a 128 x 128 tile takes for a k-block (0.33 us).  Measured
-    // over 8192 x 4096 x 1024 and 8192 x 32000 x 1024 (us per wave of tiles): 5.3 / 5.6 for 128 x 128, 8.1 / 8.9 for 128 x 256,
-    // 4.6 / 4.9 for a pair's 256 x 128, 7.2 / 7.5 for its 256 x 256: what tells them apart is the operand bytes that an SM takes
-    // from L2 per k-block (32, 48, 24, 32 KB).  Split-K (few tiles, long reduction) adds writing and reading its partial matrices
-    // at about 6 TB/s.  Planned for the device's SM count, never for the quota of the call, so the summation order (and the
-    // result, bit for bit) is the same for every quota.
-    struct Tile { int bn, cg, cost; };
-    static const Tile kTiles[] = {{128, 1, 100}, {256, 1, 155}, {128, 2, 88}, {256, 2, 136}};
-    static const Tile kNarrow[] = {{64, 1, 100}};   // outputs of at most 64 columns
-    int bn = 64, cg = 1, splits = 1;
-    double best = -1.0;
-    for (const Tile& t : kTiles) {
-        const Tile& c = N <= 64 ? kNarrow[0] : t;
-        if ((c.bn == 256 && N < 256) || (c.cg == 2 && (M <= GM_BM || tri != 0))) continue;
-        const long long tiles = batch_ll * ((M + c.cg * GM_BM - 1) / (c.cg * GM_BM)) * ((N + c.bn - 1) / c.bn);
-        const long long at_once = plan / c.cg > 0 ? plan / c.cg : 1;
-        int sp = 1;
-        if (tiles * 2 <= at_once && p.kblocks >= 8 && tri == 0) {
-            sp = (int)(at_once / tiles);
-            if (sp > p.kblocks / 4) sp = p.kblocks / 4;
-            if (sp > 16) sp = 16;
-        }
-        const double waves = (double)((tiles * sp + at_once - 1) / at_once);
-        const double cost = waves * c.cost * ((p.kblocks + sp - 1) / sp) + (sp > 1 ? (double)sp * batch_ll * M * N / 2500.0 : 0.0);
-        if (best < 0.0 || cost < best) { best = cost; bn = c.bn; cg = c.cg; splits = sp; }
-    }
+    const GemmPlan pl = gm_plan(M, N, K, batch_ll, tri, plan, num_ctas);
+    const int bn = pl.bn, cg = pl.cg;
+    int splits = pl.splits;
     p.tiles_m = (M + cg * GM_BM - 1) / (cg * GM_BM);
     p.tiles_n = (N + bn - 1) / bn;
     const long long tiles = batch_ll * p.tiles_m * p.tiles_n;
@@ -652,7 +691,7 @@ extern "C" int ob200_gemm_bf16_ex(const void* a, const void* b, void* c, const f
         }
     }
     const long long units = tiles * p.splits;
-    int grid = units * cg < num_ctas ? (int)(units * cg) : num_ctas;
+    int grid = units * cg < pl.grid ? (int)(units * cg) : pl.grid;   // fewer where the scratch took fewer splits
     // ORION_GEMM_TILES_PER_CTA=t (t > 0): a CTA retires after about t work units instead of staying for the whole launch, so
     // that the blocks of a higher-priority kernel find a free SM after a few microseconds (the grid is then wider than the
     // quota; the scheduler's cut to the quota, where it applies, still holds).

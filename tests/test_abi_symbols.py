@@ -80,3 +80,25 @@ def test_schedule_planning_host_logic(built):
                 assert tiles * splits <= max(tiles, ctas)
     # bad arguments are rejected
     assert lib.ob200_plan_schedule(0, 0, 64, 1, 1, 64, 148, None, None, None) < 0
+
+
+def _gemm_plan(lib, M, N, K, batch=1, tri=0, ctas=148):
+    out = [ctypes.c_int() for _ in range(4)]
+    lib.ob200_plan_gemm_bf16.argtypes = [ctypes.c_int] * 3 + [ctypes.c_longlong] + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_int)] * 4
+    assert lib.ob200_plan_gemm_bf16(M, N, K, batch, tri, ctas, *[ctypes.byref(o) for o in out]) == 0
+    return [o.value for o in out]
+
+
+@pytest.mark.parametrize("M,N,K", [(2048, 768, 3072), (3072, 768, 8192), (768, 3072, 8192), (2304, 768, 8192), (1232, 1024, 4096)])
+def test_gemm_plan_does_not_cut_a_reduction_whose_tiles_fill_the_device(built, M, N, K):
+    """Tiles of 128 x 128 occupy more than half of 148 SMs: a second launch and partial matrices cost more than they give."""
+    lib = ctypes.CDLL(built["liborion_kernels.so"])
+    assert _gemm_plan(lib, M, N, K)[2] == 1
+
+
+def test_gemm_plan_gives_shallow_products_single_ctas(built):
+    """A 64-deep product is bound by its tiles' way out of tensor memory, which pairs do not shorten."""
+    lib = ctypes.CDLL(built["liborion_kernels.so"])
+    assert _gemm_plan(lib, 512, 512, 64, 256)[:2] == [256, 1]
+    assert _gemm_plan(lib, 3072, 1024, 72)[1] == 1
+    assert _gemm_plan(lib, 8192, 4096, 1024)[:2] == [256, 2]   # a deep one is not
