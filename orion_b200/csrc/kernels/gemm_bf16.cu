@@ -506,7 +506,8 @@ static bool gm_make_map(unsigned char* out, const void* base, long long inner, l
 // 16.0 now; 3072 x 768 x 8192: 56.3, 33.7): where 128 x 128 tiles fill more than half of the device nothing is cut.
 //
 // The split is planned for the device's SM count, never for the quota of the call, so the summation order (and the result, bit for
-// bit) is the same for every quota.
+// bit) is the same for every quota.  Tile width and pairing do not touch the order; they are chosen again for a smaller quota, where
+// rounds are many and an odd CTA is lost to pairs (three CTAs, 3072 x 2304 x 768: 663 us in two, 348 in three).
 struct GemmPlan { int bn, cg, splits, grid; };
 struct GemmTile { int bn, cg; double kblock_us, tile_us, tail_us, launch_us; };
 static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int device_sms, int num_ctas) {
@@ -540,7 +541,17 @@ static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int devic
         const double us = price(t, (int)sp, at_once);
         if (pl.bn == 0 || us < best) { best = us; pl.bn = t.bn; pl.cg = t.cg; pl.splits = (int)sp; }
     }
-    const long long ctas = tiles_of(pl.bn, pl.cg) * pl.splits * pl.cg, most = pl.cg == 2 ? (num_ctas < 2 ? 2 : num_ctas & ~1) : num_ctas;   // whole pairs
+    if (num_ctas < device_sms) {
+        pl.bn = 0;
+        for (int i = 0; i < count; i++) {
+            const GemmTile& t = list[i];
+            const long long at_once = num_ctas / t.cg;
+            if (!fits(t) || at_once < 1) continue;
+            const double us = price(t, pl.splits, at_once);
+            if (pl.bn == 0 || us < best) { best = us; pl.bn = t.bn; pl.cg = t.cg; }
+        }
+    }
+    const long long ctas = tiles_of(pl.bn, pl.cg) * pl.splits * pl.cg, most = num_ctas / pl.cg * pl.cg;   // whole pairs
     pl.grid = (int)(ctas < most ? ctas : most);
     return pl;
 }

@@ -89,6 +89,19 @@ def _gemm_plan(lib, M, N, K, batch=1, tri=0, ctas=148):
     return [o.value for o in out]
 
 
+@pytest.mark.parametrize("M,N,K,batch,tri", [(1, 8, 8, 1, 0), (77, 768, 768, 1, 0), (129, 64, 4096, 1, 0), (600, 1024, 4096, 1, 0), (3072, 2304, 768, 1, 0),
+                                             (8192, 32000, 1024, 1, 0), (1024, 1024, 64, 32, 1), (512, 64, 512, 256, 2), (768, 768, 8192, 1, 0)])
+def test_gemm_plan_keeps_to_the_quota_and_to_one_split(built, M, N, K, batch, tri):
+    """At most `num_ctas` CTAs, pairs whole, and a split factor (the order of the sums) that no quota changes."""
+    lib = ctypes.CDLL(built["liborion_kernels.so"])
+    splits = _gemm_plan(lib, M, N, K, batch, tri)[2]
+    for ctas in list(range(1, 18)) + [33, 79, 80, 147, 148, 200]:
+        bn, cg, sp, grid = _gemm_plan(lib, M, N, K, batch, tri, ctas)
+        assert sp == splits and 1 <= grid <= ctas and grid % cg == 0
+        assert bn in ((64,) if N <= 64 else (128, 256)) and not (cg == 2 and (M <= 128 or tri)) and not (bn == 256 and N < 256)
+    assert _gemm_plan(lib, M, N, K, batch, tri, 1)[1] == 1
+
+
 @pytest.mark.parametrize("M,N,K", [(2048, 768, 3072), (3072, 768, 8192), (768, 3072, 8192), (2304, 768, 8192), (1232, 1024, 4096)])
 def test_gemm_plan_does_not_cut_a_reduction_whose_tiles_fill_the_device(built, M, N, K):
     """Tiles of 128 x 128 occupy more than half of 148 SMs: a second launch and partial matrices cost more than they give."""
@@ -102,3 +115,4 @@ def test_gemm_plan_gives_shallow_products_single_ctas(built):
     assert _gemm_plan(lib, 512, 512, 64, 256)[:2] == [256, 1]
     assert _gemm_plan(lib, 3072, 1024, 72)[1] == 1
     assert _gemm_plan(lib, 8192, 4096, 1024)[:2] == [256, 2]   # a deep one is not
+    assert _gemm_plan(lib, 3072, 2304, 768, ctas=3)[1] == 1    # two of three CTAs would work
