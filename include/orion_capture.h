@@ -51,6 +51,9 @@ int orion_capture_mark_elastic(const void* func, int ctas_per_sm);   /* func: th
 int orion_capture_quota_hint(void);                  /* quota the calling client would be granted now (0: whole device) */
 int orion_capture_last_quota(void);                  /* quota carried by the calling thread's latest grant */
 unsigned orion_capture_clamp_grid(const void* func, unsigned grid_x, int num_ctas);   /* grid width under a quota */
+/* The same for a launch in clusters of `cluster` blocks: whole clusters, at least one, which is the one case in which a launch
+ * exceeds its quota (the bfloat16 GEMM on CTA pairs under a quota of one SM that is granted after it was planned). */
+unsigned orion_capture_clamp_cluster_grid(const void* func, unsigned grid_x, unsigned cluster, int num_ctas);
 unsigned long long orion_capture_clamped_launches(void);   /* launches cut to their quota so far */
 
 #ifdef __cplusplus

@@ -127,6 +127,11 @@ unsigned clamp_grid(const void* func, unsigned grid_x, int num_ctas) {
     return (unsigned)cap;
 }
 
+unsigned whole_clusters(unsigned grid_x, unsigned granted, unsigned cluster) {
+    if (granted >= grid_x || cluster <= 1) return granted;
+    return granted < cluster ? cluster : granted / cluster * cluster;
+}
+
 static inline int64_t mono_ms() {
     struct timespec ts;
     clock_gettime(CLOCK_MONOTONIC, &ts);
@@ -378,6 +383,10 @@ int orion_capture_last_quota(void) { return tls_last_quota; }
 
 // What the launch interposers would make of a grid of `grid_x` blocks of `func` under an SM quota of `num_ctas`.
 unsigned orion_capture_clamp_grid(const void* func, unsigned grid_x, int num_ctas) { return clamp_grid(func, grid_x, num_ctas); }
+// The same for a launch in clusters of `cluster` blocks.
+unsigned orion_capture_clamp_cluster_grid(const void* func, unsigned grid_x, unsigned cluster, int num_ctas) {
+    return whole_clusters(grid_x, clamp_grid(func, grid_x, num_ctas), cluster);
+}
 
 unsigned long long orion_capture_clamped_launches(void) { return g_shared.clamped_launches.load(); }
 

@@ -36,6 +36,9 @@ void gate_end(Gate* g);
 // blocks walk the work with a gridDim.x stride, so any grid width gives the same result) are cut to
 // num_ctas x their CTAs-per-SM factor; every other kernel keeps its grid.
 unsigned clamp_grid(const void* func, unsigned grid_x, int num_ctas);
+// What a launch of `grid_x` blocks in clusters of `cluster` keeps of a grid cut to `granted`: whole clusters, and at least one,
+// the least that such a launch can have (a quota below one cluster is exceeded by it).
+unsigned whole_clusters(unsigned grid_x, unsigned granted, unsigned cluster);
 
 int client_index_of_thread();
 int client_index_of_stream(void* stream);

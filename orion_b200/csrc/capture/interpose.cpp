@@ -90,13 +90,10 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* config, const void* fu
         return real_cudaLaunchKernelExC(config, func, args);
     cudaLaunchConfig_t cfg = *config;
     cfg.stream = (cudaStream_t)g.stream;
-    const unsigned granted = clamp_grid(func, cfg.gridDim.x, g.num_ctas);
-    if (granted < cfg.gridDim.x) {   // a launch in clusters keeps whole clusters
-        unsigned cluster = 1;
-        for (unsigned i = 0; i < cfg.numAttrs; i++)
-            if (cfg.attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = cfg.attrs[i].val.clusterDim.x;
-        cfg.gridDim.x = cluster <= 1 ? granted : granted < cluster ? cluster : granted / cluster * cluster;
-    }
+    unsigned cluster = 1;
+    for (unsigned i = 0; i < cfg.numAttrs; i++)
+        if (cfg.attrs[i].id == cudaLaunchAttributeClusterDimension) cluster = cfg.attrs[i].val.clusterDim.x;
+    cfg.gridDim.x = whole_clusters(cfg.gridDim.x, clamp_grid(func, cfg.gridDim.x, g.num_ctas), cluster);
     LaunchInfo li{func, {cfg.gridDim.x, cfg.gridDim.y, cfg.gridDim.z}, {cfg.blockDim.x, cfg.blockDim.y, cfg.blockDim.z},
                   cfg.dynamicSmemBytes};
     g.launch = &li;

@@ -212,6 +212,8 @@ def ctypes_lib(path):
     lib.orion_capture_mark_elastic.argtypes = [ctypes.c_void_p, ctypes.c_int]
     lib.orion_capture_clamp_grid.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_int]
     lib.orion_capture_clamp_grid.restype = ctypes.c_uint
+    lib.orion_capture_clamp_cluster_grid.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_uint, ctypes.c_int]
+    lib.orion_capture_clamp_cluster_grid.restype = ctypes.c_uint
     return lib
 
 
@@ -399,3 +401,15 @@ def test_two_threads_of_one_client_take_turns_on_its_ring(built, tmp_path):
     r = json.loads(out.stdout.strip().splitlines()[-1])
     assert r["got"] == {"main": 30 * 20, "helper": 30 * 20, "wrong": 0}
     assert r["stats"]["hp_submits"] + r["stats"]["be_submits"] >= 30 * 40 and r["stats"]["join_timeouts"] == 0
+
+
+@pytest.mark.parametrize("quota,whole_pairs", [(1, 2), (2, 2), (3, 2), (7, 6), (147, 146), (148, 148), (0, 148)])
+def test_a_launch_in_clusters_is_cut_to_whole_clusters(built, quota, whole_pairs):
+    cap = ctypes_lib(built["liborion_capture.so"])
+    k = 0x7f0000007890
+    assert cap.orion_capture_mark_elastic(k, 1) == 0
+    assert cap.orion_capture_clamp_cluster_grid(k, 148, 2, quota) == whole_pairs
+    assert cap.orion_capture_clamp_cluster_grid(k, 148, 1, quota) == (quota or 148)
+    assert cap.orion_capture_clamp_cluster_grid(k, 2, 2, quota) == 2      # one pair already
+    assert cap.orion_capture_clamp_cluster_grid(k + 16, 148, 2, quota) == 148   # not declared elastic
+
