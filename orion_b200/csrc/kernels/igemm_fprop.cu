@@ -574,16 +574,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
         uint64_t* res_bar = &ctl->res_full[epi_id];
         uint32_t res_phase = 0;
         // The epilogue warps meet three times per piece of a cut tile, at a named barrier, which has no limit of its own.  So a
-        // warp that has given up (`ok` is false) stays in the loop and meets the others for every such piece until the work is
-        // walked; they get there too, since their own waits run out or see the abort flag.  (Bounded waits on a shared-memory
-        // barrier instead: 0.7 us more for each layer of cut tiles.)
+        // warp that has given up (`ok` is false) goes on to meet the others for every such piece until the work is walked; they
+        // get there too, since their own waits run out or see the abort flag.  (Bounded waits on a shared-memory barrier instead:
+        // 0.7 us more for each layer of cut tiles.)
         const int epi_threads = 128 * epi_groups;
         auto meet = [&] { asm volatile("bar.sync 1, %0;" ::"r"(epi_threads) : "memory"); };
         bool ok = true;
         int local = 0;
         WorkIter work(p, tiles);
         Seg seg;
-        for (; work.next(seg); local++) {
+        for (; ok && work.next(seg); local++) {
             const int tile = seg.tile;
             const int bidx = tile / tiles_per_problem;
             const int tloc = tile - bidx * tiles_per_problem;
@@ -594,12 +594,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             const uint32_t acc_use = cross ? (uint32_t)local : (uint32_t)(local >> 1);
             const long long tile_row0 = (long long)tm * BM + q * 32;
             // the residual of the first 32 columns is on its way while the tile is computed
-            if (fetch && ok && seg.nseg <= 1 && tn * BN + col_lo < p.Kout) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + col_lo);
-            if (!ok || !timed_wait_warp(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
-                ok = false;
+            if (fetch && seg.nseg <= 1 && tn * BN + col_lo < p.Kout) fetch_residual32(p, stage, res_bar, lane, tile_row0, tn * BN + col_lo);
+            if (!timed_wait_warp(&ctl->tmem_full[ab], acc_use & 1u, abort_flag, waited)) {
                 if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_FULL); }
-                if (seg.nseg > 1 && p.mode == 0) { meet(); meet(); meet(); }
-                continue;
+                ok = false;
+                break;
             }
             tc_fence_after_sync();
             if (p.mode == 1) {
@@ -711,6 +710,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                     if (tid == 0) p.counters[seg.slot] = 0;
                 }
                 meet();   // last_flag is rewritten by the next piece
+                seg.nseg = 0;   // met
                 continue;
             }
 #pragma unroll 1
@@ -738,6 +738,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
             tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) mbar_arrive(&ctl->tmem_empty[ab]);
+        }
+        if (!ok && p.mode == 0) {
+            do {
+                if (seg.nseg > 1) { meet(); meet(); meet(); }
+            } while (work.next(seg));
         }
         if (!ok && fetch) mbar_wait_landed(res_bar, res_phase);   // a residual copy may still be under way: the slab must outlive it
         if (lane == 0) bulk_wait_group_read<0>();   // the slabs must outlive the copies that read them
