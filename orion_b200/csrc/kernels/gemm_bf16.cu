@@ -507,7 +507,8 @@ static bool gm_make_map(unsigned char* out, const void* base, long long inner, l
 //
 // The split is planned for the device's SM count, never for the quota of the call, so the summation order (and the result, bit for
 // bit) is the same for every quota.  Tile width and pairing do not touch the order; they are chosen again for a smaller quota, where
-// rounds are many and an odd CTA is lost to pairs (three CTAs, 3072 x 2304 x 768: 663 us in two, 348 in three).
+// rounds are many and an odd CTA is lost to pairs (three CTAs, 3072 x 2304 x 768: 663 us in two, 348 in three).  With few CTAs at
+// work a pair's k-block gains 7 % more on a single CTA's than on the full device (seven CTAs, 8192 x 1024 x 1024: 201 us in six, 212).
 struct GemmPlan { int bn, cg, splits, grid; };
 struct GemmTile { int bn, cg; double kblock_us, tile_us, tail_us, launch_us; };
 static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int device_sms, int num_ctas) {
@@ -519,9 +520,9 @@ static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int devic
     const long long kblocks = (K + GM_BK - 1) / GM_BK;
     auto tiles_of = [&](int bn, int cg) { return batch * (((long long)M + cg * GM_BM - 1) / (cg * GM_BM)) * (((long long)N + bn - 1) / bn); };
     auto fits = [&](const GemmTile& t) { return !((t.bn == 256 && N < 256) || (t.cg == 2 && (M <= GM_BM || tri != 0))); };
-    auto price = [&](const GemmTile& t, int splits, long long at_once) {
+    auto price = [&](const GemmTile& t, int splits, long long at_once, double pair_relief) {
         const double rounds = (double)((tiles_of(t.bn, t.cg) * splits + at_once - 1) / at_once);
-        const double depth = (double)((kblocks + splits - 1) / splits) * t.kblock_us;
+        const double depth = (double)((kblocks + splits - 1) / splits) * t.kblock_us * (t.cg == 2 ? pair_relief : 1.0);
         const double us = t.launch_us + rounds * (depth > t.tile_us ? depth : t.tile_us) + t.tail_us;
         return splits > 1 ? us + 6.0 + (double)splits * batch * M * N * 8.0 / 6e6 : us;
     };
@@ -538,7 +539,7 @@ static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int devic
             if (sp > kblocks / 4) sp = kblocks / 4;
             if (sp > 16) sp = 16;
         }
-        const double us = price(t, (int)sp, at_once);
+        const double us = price(t, (int)sp, at_once, 1.0);
         if (pl.bn == 0 || us < best) { best = us; pl.bn = t.bn; pl.cg = t.cg; pl.splits = (int)sp; }
     }
     if (num_ctas < device_sms) {
@@ -547,7 +548,7 @@ static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int devic
             const GemmTile& t = list[i];
             const long long at_once = num_ctas / t.cg;
             if (!fits(t) || at_once < 1) continue;
-            const double us = price(t, pl.splits, at_once);
+            const double us = price(t, pl.splits, at_once, 0.93);
             if (pl.bn == 0 || us < best) { best = us; pl.bn = t.bn; pl.cg = t.cg; }
         }
     }
