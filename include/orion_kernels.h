@@ -72,6 +72,8 @@ int ob200_conv2d_dgrad(const void* dy, const void* wt, void* dx, int dtype, int 
  * src/scheduler/utils_sched.cpp:465-489, trapped at src/cuda_capture/intercept_cudnn.cpp:560-640). */
 int ob200_conv2d_wgrad(const void* x, const void* dy, float* dw, int dtype, int Nb, int H, int W, int C, int Kout, int R, int S,
                        int stride_h, int stride_w, int pad_h, int pad_w, int dil_h, int dil_w, int num_ctas, void* stream);
+/* Pixel ranges that a filter gradient of `tiles` 128-row tiles and `kblocks` blocks of 32 pixels is cut into (host logic only). */
+int ob200_plan_wgrad_splits(long long tiles, int kblocks, int num_ctas);
 /* w [K, R*S, C] -> wt [C, R*S, K]; elem_bytes 4 or 2.  No counterpart in the reference (cuDNN re-lays filters internally). */
 int ob200_filter_transpose(const void* w, void* wt, int K, int RS, int C, int elem_bytes, void* stream);
 

@@ -425,6 +425,22 @@ extern "C" int ob200_conv2d_dgrad(const void* dy, const void* wt, void* dx, int 
     return ob200_igemm_launch(&p, bn, grid, stream);
 }
 
+// Pixel ranges a filter gradient is cut into: two rounds of units over the granted SMs, however few the tiles (64 ranges at most left
+// more than half of the device idle on layers of one tile: MobileNetV2's 32 -> 16 at 112 x 112, batch 64, 298 us in 64 ranges, 137
+// in 296, and a fifth of the error, the truncating accumulator chains being shorter).  Every range adds its tile to dw with atomics, so
+// where that left fewer than four k-blocks to each, one round does, if that is more than 64 ranges (256 -> 64 at 56 x 56, stride 2,
+// batch 9, two tiles and 221 k-blocks: 14.1 us in 110 ranges, 11.7 in 74, 12.1 in 64).  At least two k-blocks per range.
+static int wgrad_splits(long long tiles, int kblocks, int num_ctas) {
+    long long splits = (2LL * num_ctas + tiles - 1) / tiles;
+    if (splits * 4 > kblocks && num_ctas / tiles > 64) splits = num_ctas / tiles;
+    if (splits > kblocks / 2) splits = kblocks / 2;
+    return splits < 1 ? 1 : (int)splits;
+}
+extern "C" int ob200_plan_wgrad_splits(long long tiles, int kblocks, int num_ctas) {
+    if (tiles <= 0 || kblocks <= 0 || num_ctas <= 0) return -1;
+    return wgrad_splits(tiles, kblocks, num_ctas);
+}
+
 // Filter gradient of the convolution: dw[k,r,s,c] = sum_{n,p,q} dy[n,p,q,k] * x[n, p*stride-pad+r*dil, q*stride-pad+s*dil, c].
 // float32 only (dtype 0: 3xTF32, 2: one TF32 pass); C and Kout multiples of 4.  The reduction over the
 // N*P*Q pixels is split across CTAs and summed with atomic adds, so dw is cleared on `stream` first.
@@ -471,13 +487,7 @@ extern "C" int ob200_conv2d_wgrad(const void* x, const void* dy, float* dw, int 
     p.kblocks_per_r = (int)((Mpix + 31) / 32);
     p.num_kblocks = p.kblocks_per_r;
     const long long tiles = (long long)p.tiles_m * p.tiles_n;
-    // About two units per granted SM, however few the tiles: a cap of 64 splits left more than half of the device idle on layers
-    // of one tile (MobileNetV2's 32 -> 16 at 112 x 112, batch 64: 298 -> 137 us, and a fifth of the error, the
-    // truncating accumulator chains being shorter).
-    long long splits = (2LL * num_ctas + tiles - 1) / tiles;
-    if (splits > p.num_kblocks / 2) splits = p.num_kblocks / 2;    // at least two k-blocks per unit
-    if (splits < 1) splits = 1;
-    p.splits = (int)splits;
+    p.splits = wgrad_splits(tiles, p.num_kblocks, num_ctas);
     p.status = status_word(dev);
     p.debug = g_debug;
     igemm_set_fprop(&p);
@@ -493,10 +503,7 @@ extern "C" int ob200_conv2d_wgrad(const void* x, const void* dy, float* dw, int 
         p.ctiles = 1;
         p.tiles_n = R * S;
         const long long tiles1 = (long long)p.tiles_m * p.tiles_n;
-        long long sp = (2LL * num_ctas + tiles1 - 1) / tiles1;
-        if (sp > p.num_kblocks / 2) sp = p.num_kblocks / 2;
-        if (sp < 1) sp = 1;
-        p.splits = (int)sp;
+        p.splits = wgrad_splits(tiles1, p.num_kblocks, num_ctas);
         if (p.splits > 1 && cudaMemsetAsync(dw, 0, dw_bytes, s) != cudaSuccess) return -1;
         const long long units1 = tiles1 * p.splits;
         return ob200_igemm_launch(&p, 64, units1 < num_ctas ? (int)units1 : num_ctas, stream);

@@ -116,3 +116,18 @@ def test_gemm_plan_gives_shallow_products_single_ctas(built):
     assert _gemm_plan(lib, 3072, 1024, 72)[1] == 1
     assert _gemm_plan(lib, 8192, 4096, 1024)[:2] == [256, 2]   # a deep one is not
     assert _gemm_plan(lib, 3072, 2304, 768, ctas=3)[1] == 1    # two of three CTAs would work
+
+
+def test_filter_gradient_ranges(built):
+    """Long reductions of few tiles take two rounds of the device, shorter ones one; none is cut into ranges of one k-block."""
+    lib = ctypes.CDLL(built["liborion_kernels.so"])
+    plan = lib.ob200_plan_wgrad_splits
+    plan.argtypes = [ctypes.c_longlong, ctypes.c_int, ctypes.c_int]
+    assert plan(1, 25088, 148) == 296
+    assert plan(2, 221, 148) == 74 and plan(1, 392, 148) == 148 and plan(2, 10, 148) == 5 and plan(36, 20, 148) == 9 and plan(4, 220, 148) == 74
+    for tiles in (1, 2, 3, 9, 300):
+        for kblocks in (1, 2, 7, 130, 255, 257, 1000, 30000):
+            for ctas in (1, 7, 148):
+                n = plan(tiles, kblocks, ctas)
+                assert 1 <= n <= max(1, kblocks // 2) and (n - 1) * tiles < 2 * ctas
+                assert 4 * n <= kblocks or n * tiles <= ctas or ctas // tiles <= 64
