@@ -205,7 +205,18 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
                 __syncwarp();
             }
         }
-        if (dead) attn_give_up(ctl, p.status, OB200_ERR_WAIT_FULL);
+        // The CTA's shared and tensor memory go only when no copy and no product is under way to them.  Given up at step n of item
+        // local - 1, K copies may be out up to step n + 2, V copies and score products up to n + 1, Q up to the next item.
+        const long long t0 = clock64();
+        if (dead) {
+            attn_give_up(ctl, p.status, OB200_ERR_WAIT_FULL);
+            for (uint32_t i = n; i < n + 3; i++) mbar_wait_landed(&ctl->k_full[i % AT_RING], (i / AT_RING) & 1u, t0);
+            for (uint32_t i = n; i < n + 2; i++) mbar_wait_landed(&ctl->v_full[i % AT_RING], (i / AT_RING) & 1u, t0);
+            for (uint32_t i = n; i < n + 2; i++) mbar_wait_landed(&ctl->s_full, i & 1u, t0);
+            for (uint32_t i = local - 1; i != local + 1; i++) mbar_wait_landed(&ctl->q_full, i & 1u, t0);
+        }
+        if (n > 0) mbar_wait_landed(&ctl->o_full, (n - 1) & 1u, t0);
+        __syncwarp();
     } else {
         // ------------------------------------------------------------ softmax: thread r owns query row q0 + r (tensor-memory lane r)
         const int r = warp * 32 + lane;

@@ -206,6 +206,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
                 if (++s == C::STAGES) { s = 0; ph ^= 1u; }
             }
         }
+        if (rank == 0) ring_settle(ctl->full, C::STAGES, s, ph, C::STAGES);   // the bytes of both CTAs
         // The leading CTA's commits arrive on this CTA's barriers: they must have landed before either CTA leaves.
         for (int i = 0; CG == 2 && i < C::STAGES && !dead; i++) {
             if (!mbar_wait_warp(&ctl->empty[s], ph ^ 1u, abort_flag)) break;
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
                     if (++s == C::STAGES) { s = 0; ph ^= 1u; }
                 }
             }
+            ring_settle(ctl->empty, C::STAGES, s, ph, 1);
         }
     } else {
         // ------------------------------------------------------------ epilogue: thread = output row
@@ -282,7 +284,7 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_bf16_kernel(const __grid_c
             if (gm_tile_skipped<BN>(p, tm, tn)) continue;
             const uint32_t ab = local & 1u, use = local >> 1;
             local++;
-            if (!mbar_wait(&ctl->acc_full[ab], use & 1u, abort_flag)) {
+            if (!mbar_wait_warp(&ctl->acc_full[ab], use & 1u, abort_flag)) {
                 if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_TMEM_FULL); }
                 break;
             }

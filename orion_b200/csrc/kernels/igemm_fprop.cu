@@ -744,7 +744,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 if (seg.nseg > 1) { meet(); meet(); meet(); }
             } while (work.next(seg));
         }
-        if (!ok && fetch) mbar_wait_landed(res_bar, res_phase);   // a residual copy may still be under way: the slab must outlive it
+        if (!ok && fetch) mbar_wait_landed(res_bar, res_phase, clock64());   // a residual copy may still be under way: the slab must outlive it
         if (lane == 0) bulk_wait_group_read<0>();   // the slabs must outlive the copies that read them
         if (p.debug && blockIdx.x == 0 && tid == 0) p.debug[0] = waited;
     } else if (warp == MMA_WARP) {
@@ -826,6 +826,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                 __syncwarp();
             }
         }
+        ring_settle(ctl->empty, stages, ring.s, ring.ph, 1);
         if (p.debug && blockIdx.x == 0 && lane == 0) { p.debug[1] = waited; p.debug[2] = waited2; }
     } else if (split_id >= 0) {
         // ------------------------------------------------------------ splitters (fp32 only)
@@ -854,7 +855,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                     const bool mine = turn == grp;
                     if (++turn == ngrp) turn = 0;
                     if (!mine) continue;
-                    if (!timed_wait(&ctl->raw_full[s], ring.ph, abort_flag, waited)) {
+                    if (!timed_wait_warp(&ctl->raw_full[s], ring.ph, abort_flag, waited)) {
                         if (!*abort_flag) { ctl->abort_flag = 1; if (p.status) atomicExch(p.status, OB200_ERR_WAIT_FULL); }
                         dead = true;
                         break;
@@ -1258,6 +1259,8 @@ auto split_row = [&](auto load4) {   // load4(i): values 4i .. 4i+3 of this thre
                 }
             }
         }
+        if (tma_roles) ring_settle(ctl->raw_full, stages, ring.s, ring.ph, stages);
+        else asm volatile("cp.async.wait_all;" ::: "memory");
     }
 
     if (p.debug && blockIdx.x == 0) {

@@ -81,12 +81,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     }
 }
 
-// For a role that gives up with copies of its own under way: they must land before the CTA leaves its shared memory.  Bounded, but
-// blind to the abort flag, which is up already.
-__device__ __forceinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity) {
-    const long long t0 = clock64();
+// For a role that leaves with copies or MMAs of its own under way: they must be done before the CTA gives up its shared and tensor
+// memory.  Bounded by the same limit, counted from t0 = clock64() for all that a role waits for, but blind to the abort flag, which
+// may be up already.
+__device__ __forceinline__ void mbar_wait_landed(uint64_t* bar, uint32_t parity, long long t0) {
     while (!mbar_try_wait_hint(bar, parity, 4000u))
         if (clock64() - t0 > OB200_WAIT_CYCLES) return;
+}
+// The same for a ring of stages, (s, ph) being the position after the last stage used: the newest phases of the last `back` stages.  A
+// producer passes the barriers its copies land on, the MMA issuer (one stage back: a commit covers all MMAs before it) those its
+// commits arrive on.  A stage never used counts as done (the phase before its barrier's first).
+__device__ __forceinline__ void ring_settle(uint64_t* bars, int stages, int s, uint32_t ph, int back) {
+    const long long t0 = clock64();
+    for (int i = 0; i < back; i++) {
+        if (s == 0) { s = stages; ph ^= 1u; }
+        mbar_wait_landed(&bars[--s], ph, t0);
+    }
+    __syncwarp();
 }
 
 // The same for a whole converged warp: every lane gets the same answer, so that a wait which runs out unwinds the warp as one.

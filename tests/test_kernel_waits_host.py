@@ -58,3 +58,65 @@ def test_an_epilogue_warp_that_gives_up_keeps_meeting_the_others():
             elif ch == "}":
                 opened.pop()
         assert any("for (" in h for h in opened) or walk[:m.start()].rstrip().endswith("ok = false;")
+
+
+SHIM = """
+#include <cstdint>
+static int waited[64][2], waits;
+static inline void mbar_wait_landed(uint64_t* bar, uint32_t parity, long long) { waited[waits][0] = (int)*bar; waited[waits++][1] = (int)parity; }
+static inline void __syncwarp() {}
+static inline long long clock64() { return 0; }
+#define __device__
+#define __forceinline__ inline
+%s
+extern "C" int settle(int stages, int used, int back, int* out) {
+    uint64_t bars[16];
+    for (int i = 0; i < stages; i++) bars[i] = i;
+    waits = 0;
+    ring_settle(bars, stages, used %% stages, (uint32_t)(used / stages) & 1u, back);
+    for (int i = 0; i < waits; i++) { out[2 * i] = waited[i][0]; out[2 * i + 1] = waited[i][1]; }
+    return waits;
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def settle(tmp_path_factory):
+    import ctypes
+    import subprocess
+    text = open(os.path.join(KERNELS, "sm100_primitives.cuh")).read()
+    start = text.index("__device__ __forceinline__ void ring_settle")
+    func = text[start:text.index("{", start)] + "{" + _block(text, start) + "}"
+    d = tmp_path_factory.mktemp("settle")
+    (d / "settle.cpp").write_text(SHIM % func)
+    subprocess.run(["g++", "-shared", "-fPIC", "-std=c++17", "-o", str(d / "settle.so"), str(d / "settle.cpp")], check=True)
+    fn = ctypes.CDLL(str(d / "settle.so")).settle
+
+    def call(stages, used, back):
+        out = (ctypes.c_int * 128)()
+        n = fn(stages, used, back, out)
+        return [(out[2 * i], out[2 * i + 1]) for i in range(n)]
+    return call
+
+
+@pytest.mark.parametrize("stages", [1, 2, 3, 4, 6, 8])
+def test_a_role_that_leaves_waits_for_the_last_lap_of_its_ring(settle, stages):
+    """After `used` uses of the ring: the newest phase of every stage (use n of a stage is its barrier's phase n // stages), and for a
+    stage never used the phase before the first, which counts as complete."""
+    for used in range(0, 4 * stages + 1):
+        want = {s: (max(n // stages for n in range(used) if n % stages == s) & 1 if used > s else 1) for s in range(stages)}
+        assert dict(settle(stages, used, stages)) == want and len(settle(stages, used, stages)) == stages
+        last = (used - 1) % stages
+        assert settle(stages, used, 1) == [(last, want[last])]
+
+
+@pytest.mark.parametrize("name,copies,products", [("igemm_fprop.cu", ["ctl->raw_full"], ["ctl->empty"]), ("gemm_bf16.cu", ["ctl->full"], ["ctl->empty"]),
+                                                  ("attention.cu", ["&ctl->k_full", "&ctl->v_full", "&ctl->q_full"], ["&ctl->s_full", "&ctl->o_full"])])
+def test_roles_leave_with_no_copy_and_no_product_under_way(name, copies, products):
+    """On every way out of a role, given up or not, what it set off has landed (or a bounded wait for it has run out) before the CTA's
+    shared and tensor memory go."""
+    roles = _roles(name)
+    for bar in copies + products:
+        assert re.search(r"(ring_settle|mbar_wait_landed)\(" + re.escape(bar), roles), bar
+    # a warp-wide instruction behind a wait needs the same answer in all lanes
+    assert not re.search(r"if \(!(dead && !)?mbar_wait\(|!timed_wait\(&ctl->(raw_full|tmem)", roles)
