@@ -215,10 +215,9 @@ int ob200_softmax_causal(const void* x, void* y, long long rows, int D, float sc
  * (reference src/scheduler/utils_sched.cpp:502-513). */
 int ob200_attention_fwd_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal, int num_ctas,
                              void* stream);
-/* The same for any S; lse (float [B, H, S], may be NULL) receives per query the base-2 logarithm of the sum over its keys of
- * exp(scaled score).  One call computes part `part` of `parts` of the query tiles (0, 1: all of them). */
-int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* lse, int B, int S, int H, int head_dim, float scale, int causal,
-                                 int part, int parts, int num_ctas, void* stream);
+/* The same for any S.  One call computes part `part` of `parts` of the query tiles (0, 1: all of them). */
+int ob200_attention_long_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal, int part, int parts,
+                              int num_ctas, void* stream);
 
 /* Training side of the transformer clients (dtype 0 float32, 1 bfloat16; parameters in the activations' type).  They
  * stand in for the kernels the reference's BERT training profile lists (reference benchmarking/model_kernels/bert_8_fb1:

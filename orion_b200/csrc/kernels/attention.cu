@@ -38,7 +38,6 @@ constexpr float AT_RESCALE = 8.f;   // the reference maximum moves when a row's 
 
 struct AttnParams {
     void* ctx;             // [B, S, H*64] bfloat16
-    float* lse;            // [B, H, S] log2 of the sum over the keys of 2^(scaled score * log2 e), or null
     int* status;
     int B, S, H;
     int causal;
@@ -334,7 +333,6 @@ __global__ void __launch_bounds__(AT_THREADS, AT_CTAS_PER_SM) attention_fwd_kern
                     }
                 }
             }
-            if (p.lse && qpos < p.S) p.lse[((long long)it.b * p.H + it.h) * p.S + qpos] = m_ref + log2f(sum);
             tc_fence_before_sync();   // the next item's first product overwrites O only behind its p_full
         }
         if (!ok) attn_give_up(ctl, p.status, OB200_ERR_WAIT_TMEM_FULL);
@@ -367,8 +365,8 @@ extern "C" int* ob200_status_word_for_current_device(void);
 
 // See include/orion_kernels.h.  Returns -1 for unsupported sizes, -2 for misaligned pointers, -4 when the TMA descriptor cannot
 // be built.
-extern "C" int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* lse, int B, int S, int H, int head_dim, float scale, int causal,
-                                            int part, int parts, int num_ctas, void* stream) {
+extern "C" int ob200_attention_long_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal, int part,
+                                         int parts, int num_ctas, void* stream) {
     using namespace ob200;
     if (B <= 0 || S <= 0) return 0;
     if (head_dim != AT_D || H <= 0 || num_ctas <= 0 || parts < 1 || part < 0 || part >= parts) return -1;
@@ -378,7 +376,6 @@ extern "C" int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* l
     AttnParams p;
     memset(&p, 0, sizeof p);
     p.ctx = ctx;
-    p.lse = lse;
     p.status = ob200_status_word_for_current_device();
     p.B = B; p.S = S; p.H = H;
     p.causal = causal ? 1 : 0;
@@ -434,5 +431,5 @@ extern "C" int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* l
 extern "C" int ob200_attention_fwd_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal,
                                         int num_ctas, void* stream) {
     if (B > 0 && S > 384) return -1;
-    return ob200_attention_fwd_lse_bf16(qkv, ctx, nullptr, B, S, H, head_dim, scale, causal, 0, 1, num_ctas, stream);
+    return ob200_attention_long_bf16(qkv, ctx, B, S, H, head_dim, scale, causal, 0, 1, num_ctas, stream);
 }

@@ -80,8 +80,8 @@ int ob200_embedding_backward(const void* dy, const long long* ids, long long per
                              long long tokens, int D, int dtype, int num_ctas, void* stream);
 int ob200_attention_fwd_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal, int num_ctas,
                              void* stream);
-int ob200_attention_fwd_lse_bf16(const void* qkv, void* ctx, float* lse, int B, int S, int H, int head_dim, float scale, int causal,
-                                 int part, int parts, int num_ctas, void* stream);
+int ob200_attention_long_bf16(const void* qkv, void* ctx, int B, int S, int H, int head_dim, float scale, int causal, int part, int parts,
+                              int num_ctas, void* stream);
 int ob200_layernorm_train_forward(const void* x, void* y, const void* gamma, const void* beta, float* mean, float* rstd, long long rows,
                                   int D, float eps, int dtype, int num_ctas, void* stream);
 int ob200_layernorm_backward(const void* dy, const void* x, const void* gamma, const float* mean, const float* rstd, void* dx,
@@ -507,9 +507,9 @@ at::Tensor attention_long_op(const at::Tensor& qkv, int64_t heads, double scale,
     at::Tensor ctx = at::empty({qkv.size(0) * qkv.size(1), heads * 64}, qkv.options());
     constexpr int kParts = 3;
     for (int part = 0; part < kParts; part++)
-        check(ob200_attention_fwd_lse_bf16(qkv.data_ptr(), ctx.data_ptr(), nullptr, (int)qkv.size(0), (int)qkv.size(1), (int)heads, 64,
-                                           (float)scale, causal ? 1 : 0, part, kParts, quota(), cur_stream()),
-              "ob200_attention_fwd_lse_bf16");
+        check(ob200_attention_long_bf16(qkv.data_ptr(), ctx.data_ptr(), (int)qkv.size(0), (int)qkv.size(1), (int)heads, 64, (float)scale,
+                                        causal ? 1 : 0, part, kParts, quota(), cur_stream()),
+              "ob200_attention_long_bf16");
     return ctx;
 }
 
