@@ -6,8 +6,9 @@
 // and no re-laid-out Q / K / V copies in HBM.  It stands in for the two cublasSgemmStridedBatched calls around a softmax
 // kernel that the reference replays for an attention layer (reference src/scheduler/utils_sched.cpp:502-513).
 //
-// One work item = 128 query rows of one (batch, head); a persistent grid walks the items, 64 keys a step with a running
-// maximum.  Bound: the exponentials (16 per clock and SM; the two products of a step take a third of that time), so what
+// One work item = 128 query rows of one (batch, head); a persistent grid walks the items, 64 keys a step by the online softmax
+// (Milakov and Gimelshein, 2018): sums and output are relative to a running reference maximum, here one that moves only when a
+// row's maximum has outgrown it by 2^8.  Bound: the exponentials (16 per clock and SM; the two products of a step take a third of that time), so what
 // counts is that twelve softmax warps per SM always have scores to work on: scores and output of one item take 128
 // tensor-memory columns and 66 KB of shared memory, and three items share an SM.
 // 8 x 384 x 12 heads: 33.1 us with all scores of a query tile in tensor memory (one item per SM, two passes over them), 15.0 now;
@@ -33,7 +34,7 @@ constexpr int AT_THREADS = 192;     // warps 0-3: softmax / epilogue (one thread
 constexpr int AT_Q_BYTES = AT_QROWS * 128, AT_KV_BYTES = AT_KEYS * 128, AT_P_BYTES = AT_QROWS * 128;
 constexpr int AT_RING = 2;          // K tiles and V tiles in flight
 constexpr int AT_SMEM = AT_Q_BYTES + 2 * AT_RING * AT_KV_BYTES + AT_P_BYTES + 1024 + 256;   // + alignment, barriers
-constexpr int AT_CTAS_PER_SM = 3;   // 66 KB of shared memory, 128 tensor-memory columns and 112 registers per thread each
+constexpr int AT_CTAS_PER_SM = 3;   // 66 KB of shared memory, 128 tensor-memory columns and at most 112 registers per thread each
 constexpr float AT_RESCALE = 8.f;   // the reference maximum moves when a row's maximum outgrows it by 2^8
 
 struct AttnParams {

@@ -140,7 +140,6 @@ __global__ void __launch_bounds__(ELT_THREADS) maxpool_nhwc_f32_kernel(const flo
 __global__ void __launch_bounds__(ELT_THREADS) maxpool3x3s2_nhwc_f32_kernel(const float* __restrict__ x, float* __restrict__ y,
                                                                           int Nb, int H, int W, int C, int P, int Q, int pad) {
     pdl_wait();
-    pdl_launch_dependents();
     pdl_launch_dependents();   // a convolution behind this kernel may set itself up meanwhile (pdl.cuh)
     const int c4 = C >> 2, qb_n = (Q + 3) / 4;
     const long long total = (long long)Nb * P * qb_n * c4;

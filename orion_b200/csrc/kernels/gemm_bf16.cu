@@ -13,8 +13,8 @@
 // One CTA = 128 x BN output tile per work unit, persistent over units; or a pair of CTAs (a cluster on the two SMs of a TPC,
 // cta_group::2) = 256 x BN, each CTA staging its 128 rows of A and half of B, so that an SM takes 32 KB instead of 48 KB of
 // operands from L2 per 128 x 256 x 64 product of its own.  Operand traffic is what bounds the single CTA (about 64 bytes a clock
-// and SM): decoder feed-forward 8192 x 4096 x 1024 56.6 -> 50.2 us (1.37 PFLOP/s), vocabulary projection 8192 x 32000 x 1024
-// 487 -> 411 us.  Warp 0 issues TMA copies (4-D tensor maps:
+// and SM): decoder feed-forward 8192 x 4096 x 1024 57.9 -> 50.3 us (1.37 PFLOP/s), vocabulary projection 8192 x 32000 x 1024
+// 505 -> 411 us.  Warp 0 issues TMA copies (4-D tensor maps:
 // inner, outer, batch_inner, batch_outer; out-of-range elements read as zero, so ragged M, N, K need no special path),
 // warp 1 issues tcgen05.mma kind::f16 into one of two tensor-memory accumulators, warps 2-5 drain the other one:
 // tcgen05.ld (one output row per thread), alpha / bias / residual in registers, 32 rows x 128 bytes staged in a swizzled

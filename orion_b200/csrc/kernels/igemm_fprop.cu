@@ -55,10 +55,11 @@ constexpr int EPI_WARPS = 4;      // warps 0-3; TMA-fed launches add warps 9-12 
 constexpr int MMA_WARP = 4;
 constexpr int SPLIT_WARPS = 4;    // warps 5-8; TMA-fed launches add warps 13-16 as a second splitter group
 constexpr int PROD_WARPS = 8;     // warps 9-16 when the operands are gathered with cp.async
-constexpr int TMA_WARP = 17;      // one lane issues the TMA copies of TMA-fed launches
+constexpr int TMA_WARP = 17;      // TMA-fed launches: runs as one warp, an elected lane issues the copies
 constexpr int NTHREADS = 18 * 32;
 
-// ATMEM: 3xTF32 with both parts of the activation tile in tensor memory (the activation of forward, data gradient and GEMM, dy of a TMA-fed filter gradient).
+// ATMEM: 3xTF32 with both parts of the first operand's tile in tensor memory (the activation of forward, data gradient and GEMM,
+// dy of a TMA-fed filter gradient).
 template <typename T, int BN, int PASSES, bool ATMEM>
 struct Cfg {
     static constexpr bool kSplit = sizeof(T) == 4 && PASSES == 3;   // 3xTF32; PASSES == 1 is plain TF32
@@ -872,7 +873,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) igemm_fprop_kernel(const __grid_c
                         const int q = warp & 3;
                         const uint32_t row = (uint32_t)(q * 32 + lane);
                         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + C::A_TMEM_COL0 + s * 64;
-auto split_row = [&](auto load4) {   // load4(i): values 4i .. 4i+3 of this thread's row
+                        auto split_row = [&](auto load4) {   // load4(i): values 4i .. 4i+3 of this thread's row
 #pragma unroll
                             for (int c0 = 0; c0 < 32; c0 += 16) {
                                 uint32_t hi[16], lo[16];

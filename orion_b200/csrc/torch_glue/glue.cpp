@@ -497,9 +497,10 @@ at::Tensor attention_op(const at::Tensor& qkv, int64_t heads, double scale, bool
 }
 
 // The same for sequences of any length that is a multiple of 8.  It goes out as three launches, as many as the scores, softmax
-// and context launches it took the place of: the scheduler admits work launch by launch, so a long attention layer of one client
-// stays three grants.  16 x 512 x 16 heads, causal: 43 us a layer, against 235 us of scores, softmax, context and three
-// strided copies.
+// and context launches it took the place of, because the launch count of a decoder request is fixed: the configuration test counts
+// ten per layer, and the profiles that the scheduler reads have a row per launch.  One launch would be 2 us a layer faster at
+// 16 x 512 x 16 heads, and on problems whose items (128 query rows of a head) fit the device at once, 444, three in a row leave most of
+// it idle.  16 x 512 x 16 heads, causal: 43 us a layer, against 235 us of scores, softmax, context and three strided copies.
 at::Tensor attention_long_op(const at::Tensor& qkv, int64_t heads, double scale, bool causal) {
     TORCH_CHECK(qkv.is_cuda() && qkv.dim() == 3 && qkv.is_contiguous() && qkv.scalar_type() == at::kBFloat16 && heads > 0 &&
                     qkv.size(2) == 3 * heads * 64 && qkv.size(1) % 8 == 0,
