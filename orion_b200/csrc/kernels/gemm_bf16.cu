@@ -502,7 +502,9 @@ static bool gm_make_map(unsigned char* out, const void* base, long long inner, l
 // memory, whichever is longer, the way out of the last one, and for pairs the start of a launch in clusters.  Split-K (few tiles,
 // long reduction) adds the second launch and writing and reading the partial matrices at about 6 TB/s.  The constants are a fit
 // to 359 shapes (16 - 8192 tokens times the widths of the clients' layers in all three layouts, and batched attention products),
-// each measured in every tiling: the choice is 0.3 % slower than the fastest tiling of the same split on average, 7 % at worst.
+// each measured in every tiling, warm and back to back: the choice is 0.4 % slower than the fastest tiling of the same split on
+// average, 7 % at worst.  That fit alone would have put the start of a launch in clusters at 1.8; in the models, where weights come
+// from HBM, pairs gain more: BERT request 8 x 384 1466 us at 1.2 and below, 1522 at 1.8.
 // A model of k-blocks alone took pairs where the way out bounds (64-deep products 512 x 512 x 256 problems: 54.2 us, 43.3 in single
 // CTAs; 3072 x 1024 over 72 tokens 6.9, 6.2) and cut reductions that one round of 128-wide tiles had held (2048 x 768 x 3072: 34.5 us,
 // 16.0 now; 3072 x 768 x 8192: 56.3, 33.7): where 128 x 128 tiles fill more than half of the device nothing is cut.
@@ -516,7 +518,7 @@ struct GemmTile { int bn, cg; double kblock_us, tile_us, tail_us, launch_us; };
 static GemmPlan gm_plan(int M, int N, int K, long long batch, int tri, int device_sms, int num_ctas) {
     static const GemmTile kNarrow = {64, 1, 0.44, 2.15, 1.0, 0.0};   // outputs of at most 64 columns
     static const GemmTile kTiles[] = {{128, 1, 0.44, 2.15, 1.0, 0.0}, {256, 1, 0.51, 3.0, 2.0, 0.0},
-                                      {128, 2, 0.32, 2.15, 1.0, 1.8}, {256, 2, 0.45, 3.0, 2.0, 1.8}};
+                                      {128, 2, 0.32, 2.15, 1.0, 1.3}, {256, 2, 0.45, 3.0, 2.0, 1.3}};
     const GemmTile* list = N <= 64 ? &kNarrow : kTiles;
     const int count = N <= 64 ? 1 : 4;
     const long long kblocks = (K + GM_BK - 1) / GM_BK;
