@@ -69,6 +69,33 @@ def test_tiles_of_cta_pairs_at_their_edges(built, trans_a, trans_b, M, N, K):
     assert K_.read_status() == 0
 
 
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("M,N,K,tile,split", [(1030, 1000, 520, 128, False), (3100, 264, 776, 128, False), (520, 1000, 2056, 128, True),
+                                              (1000, 264, 4104, 128, True), (1030, 4100, 1032, 256, False), (1000, 1000, 8200, 256, True)])
+def test_launches_in_pairs_at_their_edges(built, trans_a, trans_b, M, N, K, tile, split):
+    """Shapes that the plan gives to pairs of CTAs: rows that end in the first or in the second CTA of the last pair, ragged columns and
+    reductions; the same bits from CTA counts that take pairs, single CTAs and other tile widths."""
+    import ctypes
+    from orion_b200 import kernels as K_
+    L = K_.lib()
+    out = [ctypes.c_int() for _ in range(4)]
+    L.ob200_plan_gemm_bf16.argtypes = [ctypes.c_int] * 3 + [ctypes.c_longlong] + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_int)] * 4
+    assert L.ob200_plan_gemm_bf16(M, N, K, 1, 0, 148, *[ctypes.byref(o) for o in out]) == 0
+    assert out[0].value == tile and out[1].value == 2 and (out[2].value > 1) == split
+    torch.manual_seed(M + N + K)
+    def mat(rows, cols):
+        ld = (cols + 7) // 8 * 8
+        return torch.randn(rows, ld, device="cuda").to(torch.bfloat16)[:, :cols]
+    a = mat(K, M) if trans_a else mat(M, K)
+    b = mat(K, N) if trans_b else mat(N, K)
+    ref = _ref(a, b, trans_a, trans_b, None, 1.0)
+    outs = [K_.gemm_bf16(a, b, trans_a, trans_b, out_dtype=torch.float32, num_ctas=n) for n in (148, 40, 3, 1)]
+    _check(outs[0], ref, K)
+    assert all(torch.equal(outs[0], o) for o in outs[1:])
+    _check(K_.gemm_bf16(a, b, trans_a, trans_b), ref, K)
+    assert K_.read_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(768, 768, 3072), (2304, 768, 3072), (1024, 1024, 8192), (768, 136, 2000)])
 def test_weight_gradient_shapes_take_split_k_and_do_not_depend_on_the_cta_count(built, M, N, K):
     """dW = dY^T . X: both operands [tokens, features]; few output tiles and a long reduction."""
