@@ -42,10 +42,10 @@ def test_an_epilogue_warp_that_gives_up_keeps_meeting_the_others():
     roles = _roles("igemm_fprop.cu")
     epilogue = _block(roles, roles.index("if (epi_id >= 0)"))
     head = re.search(r"for \(; ([^;]*); local\+\+\)", epilogue)
-    assert head.group(1) == "ok && work.next(seg)"
+    assert head.group(1) == "__builtin_expect(ok, 1) && work.next(seg)"
     walk = _block(epilogue, head.end())
     behind = epilogue[epilogue.index(walk) + len(walk):]
-    given_up = _block(behind, behind.index("if (!ok && p.mode == 0)"))
+    given_up = _block(behind, behind.index("if (__builtin_expect(!ok, 0) && p.mode == 0)"))
     assert re.match(r"\s*do \{\s*if \(seg\.nseg > 1\)", given_up) and given_up.rstrip().endswith("while (work.next(seg));")
     assert given_up.count("meet()") == walk.count("meet()") == 3 and "return" not in walk
     # left with the piece's own three meetings behind it only where it says so
